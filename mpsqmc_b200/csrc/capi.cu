@@ -96,11 +96,15 @@ struct mpsqmc_ctx {
   long scr_base = 0;                    // scratch doubles per CTA before the matrix work buffers
   long all_doubles = 0, big_doubles = 0;  // work buffers: all of them / the matrix ones
   long mlp_doubles = 0;                 // the learned proposal's small buffers (on chip while it is in use)
-  size_t smem_optin = 0;
+  size_t smem_optin = 0, smem_sm = 0, total_mem = 0;  // of the device: shared memory of a CTA, of an SM; memory
   bool global_work = false;             // matrix work buffers in global scratch
   int maxA = 1, maxB = 1, pa = 4, pb = 4, pq = 4;
   size_t smem_bytes = 0;
-  size_t smem_bytes_noqr = 0;           // the QR-free general sweep's (no Householder buffers)
+  // the QR-free FP64 sweep: buffer placement, dynamic shared memory, threads and grid
+  mq::FreeLayout fl{};
+  size_t smem_bytes_free = 0;
+  long fwoff = 0;
+  int free_threads = mq::kThreads, max_ctas_free = 1;
   int sm_count = 1, max_ctas = 1;
   // mixed-precision sweep (FP32 work buffers, TF32 tensor cores): its own shared memory and grid
   int precision = MPSQMC_PRECISION_FP64;
@@ -262,6 +266,8 @@ mq::Dev make_dev(mpsqmc_ctx *c) {
   p.eopen = c->d_eopen;
   p.choff = c->choff;
   p.gwoff = c->gwoff;
+  p.fl = c->fl;
+  p.fwoff = c->fwoff;
   p.wdims = c->d_wdims;
   p.wofs = c->d_wofs;
   p.ctr = c->d_ctr;
@@ -305,7 +311,8 @@ int canon_every(const mpsqmc_ctx *c) { return c->canon_interval > 0 ? c->canon_i
 // Doubles of per-CTA scratch for the largest grid of any walker kernel (the mixed sweep reads a
 // CTA's scratch as floats with the same stride).
 size_t scratch_doubles(const mpsqmc_ctx *c) {
-  return std::max((size_t)c->max_ctas * c->scr_stride, ((size_t)c->max_ctas_mixed * c->scr_stride + 1) / 2);
+  return std::max((size_t)std::max(c->max_ctas, c->max_ctas_free) * c->scr_stride,
+                  ((size_t)c->max_ctas_mixed * c->scr_stride + 1) / 2);
 }
 
 int layout_workspace(mpsqmc_ctx *c, bool force_global);
@@ -381,6 +388,73 @@ bool mlp_on(const mpsqmc_ctx *c) {
          (c->proposal == MPSQMC_PROPOSAL_LEARNED || c->prop_train);
 }
 
+// The QR-free FP64 sweep's threads per walker and walkers per SM.  A walker's sweep is a dependent chain of
+// small operations, so walkers that share an SM fill one another's waits; more threads per walker
+// only pay where its products fill them, or where there is no second walker for the SM.  128
+// registers a thread: 512 threads per SM.  Measured (ms per step, threads x walkers per SM):
+//   D_T = 4, D_W = 2, 1000 walkers (L = 20 chain):      256x1 2.84   128x4 0.95   64x8 0.60
+//   16, 8, 740 walkers (6x3 lattice):                   256x1 6.02   128x3 3.27   64x8 3.74
+//   64, 32, 1024 walkers (L = 64 chain):                512x1 32.1   256x2 24.8   128x3 31.6
+//   64, 32, 444 walkers (8x8 lattice):                  512x1 107    256x2 96     128x3 82
+//   64, 16-64, 444 walkers (6x6 lattice):               512x1 69     256x2 60     128x3 77
+//   16, 16, 128 walkers (L = 16 chain, one per SM):     512x1 0.50   256x1 0.42   128x1 0.55
+//   256, 64, 148 walkers (8x8 lattice, one per SM):     512x1 503    256x1 716
+void free_shape(const mpsqmc_ctx *c, int *threads, int *ctas) {
+  const long a = (long)c->maxA * c->maxB;
+  const int per_sm = std::max(1, (c->Ndesired + c->sm_count - 1) / c->sm_count);
+  int th = 512, n = 1;
+  if (a <= 64) th = 64, n = 8;
+  else if (a < 2048 || (a < 4096 && !c->nn)) th = 128, n = 3;
+  else if (a < 16384) th = 256, n = 2;
+  if (per_sm < n) {  // fewer walkers than places: more threads for each
+    n = per_sm;
+    while (2 * th * n <= 512 && (2 * th <= 256 || a >= 2048)) th *= 2;
+  }
+  *threads = th;
+  *ctas = n;
+}
+
+// That sweep's buffers (layout_workspace's part for it).  The matrix buffers go to shared memory in the
+// order of their use as right factors of products, as far as the share of a CTA reaches (with
+// room for more products at a time where all of them fit); a CTA's global scratch holds the rest.
+int layout_free(mpsqmc_ctx *c, bool force_global) {
+  int threads = 0, ctas = 0;
+  free_shape(c, &threads, &ctas);
+  const size_t share =
+      force_global ? 0 : std::min(c->smem_optin, c->smem_sm / ctas - 1024 - mq::kOpBytes);
+  auto bytes = [&](const mq::FreeLayout &f, long *big) {
+    return sizeof(double) * (size_t)mq::free_doubles(c->L, c->nC, c->maxB, c->G, c->nJ, c->pa, c->pb, f, nullptr, nullptr,
+                                                     nullptr, big);
+  };
+  const unsigned every = (1u << mq::kNumBuf) - 1;
+  mq::FreeLayout f{0u, 2};
+  for (int nx : {8, 6, 4})
+    if (!f.place && bytes({every, nx}, nullptr) <= share) f = {every, nx};
+  if (!f.place)
+    for (int k = 0; k < mq::kNumBuf; ++k) {
+      const mq::FreeLayout g{f.place | 1u << k, 2};
+      if (bytes(g, nullptr) <= share) f = g;
+    }
+  c->fl = f;
+  long big = 0;
+  c->smem_bytes_free = bytes(f, &big);
+  if (c->smem_bytes_free > c->smem_optin)
+    return fail(MPSQMC_E_UNSUPPORTED, "grid too large for the shared-memory budget of one CTA");
+  c->fwoff = (c->scr_base + 31) & ~31L;
+  c->scr_stride = std::max(c->scr_stride, (c->fwoff + big + 31) & ~31L);
+  for (const void *k : {(const void *)mq::walker_step_kernel_fp64<true>, (const void *)mq::walker_step_kernel_fp64<false>,
+                        (const void *)mq::energy_general_kernel})
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_bytes_free));
+  c->free_threads = threads;
+  int occ = 1;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mq::walker_step_kernel_fp64<false>, threads, c->smem_bytes_free));
+  // several walkers per SM only where their scratch leaves most of the device memory to the populations
+  int n = std::max(1, std::min(occ, ctas));
+  while (n > 1 && (size_t)n * c->sm_count * c->scr_stride * sizeof(double) > c->total_mem / 16) --n;
+  c->max_ctas_free = n * c->sm_count;
+  return 0;
+}
+
 int layout_workspace(mpsqmc_ctx *c, bool force_global) {
   const bool mlp = mlp_on(c);
   const long all = c->all_doubles + (mlp ? c->mlp_doubles : 0);
@@ -394,23 +468,20 @@ int layout_workspace(mpsqmc_ctx *c, bool force_global) {
     c->smem_bytes = sizeof(double) * (size_t)(all - c->big_doubles);
   }
   c->global_work = global;
-  c->smem_bytes_noqr = global ? c->smem_bytes
-                              : sizeof(double) * (size_t)mq::smem_doubles(c->L, c->maxA, c->maxB, c->G, c->pa, c->pb,
-                                                                          c->pq, nullptr, nullptr, nullptr, nullptr,
-                                                                          mlp, false);
   if (c->smem_bytes > c->smem_optin)
     return fail(MPSQMC_E_UNSUPPORTED, "grid too large for the shared-memory budget of one CTA");
   const void *kernels[] = {(const void *)mq::walker_step_kernel, (const void *)mq::set_overlap_kernel,
-                           (const void *)mq::energy_kernel, (const void *)mq::walker_step_general_kernel<true, 1>,
-                           (const void *)mq::walker_step_general_kernel<true, 1, false>,
-                           (const void *)mq::walker_step_general_kernel<true, 2>,
-                           (const void *)mq::walker_step_general_kernel<false, 0>,
-                           (const void *)mq::energy_general_kernel, (const void *)mq::legacy_step_kernel};
+                           (const void *)mq::energy_kernel, (const void *)mq::walker_step_general_kernel<true>,
+                           (const void *)mq::walker_step_general_kernel<false>, (const void *)mq::legacy_step_kernel};
   for (const void *k : kernels)
     CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_bytes));
   int occ = 1;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mq::walker_step_kernel, mq::kThreads, c->smem_bytes));
   c->max_ctas = std::max(1, occ) * c->sm_count;
+  {
+    const int rc = layout_free(c, force_global);
+    if (rc) return rc;
+  }
   // mixed-precision sweep: FP32 matrix buffers next to the small FP64 ones, on chip unless the
   // FP64 buffers were placed in global scratch
   long big_floats = 0;
@@ -486,48 +557,63 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
   for (int i = 0; i < L; ++i) site_c0[i + 1] += site_c0[i];
   // Energy channels: a site i is open on the cut before site k when it couples to some j >= k.
   // Site k closes the couplings (i, k) and opens its own channel if it has a partner beyond k.
-  // A slot freed on site k can be taken by the channel site k opens (the kernel reads closing
-  // channels before it writes the new one).
+  // A slot freed on site k is taken by a channel opened beyond k at the earliest in the per-walker
+  // sweeps, which write the opened channel before they read the closing ones; the walker-batched
+  // sweep reads first and reuses the slot on site k itself.
   std::vector<int> last_partner(L, -1);
   for (int c = 0; c < cfg->nC; ++c) last_partner[cfg->ci[c]] = std::max(last_partner[cfg->ci[c]], cfg->cj[c]);
-  std::vector<int> ech_off(L + 1, 0), ech_slot, ech_cont, eopen(L, -1), slot_of_site(L, -1), free_slots;
+  std::vector<int> ech_off, ech_slot, ech_cont, eopen;
   std::vector<double> ech_J;
-  std::vector<int> open_sites;
   int nslots = 0;
-  for (int k = 0; k < L; ++k) {
-    ech_off[k] = (int)ech_slot.size();
-    std::vector<int> still;
-    for (int i : open_sites) {
-      double J = 0.0;
-      for (int c = site_c0[i]; c < site_c0[i + 1]; ++c)
-        if (cp_j[c] == k) J += cfg->cJ[c];
-      const bool cont = last_partner[i] > k;
-      ech_slot.push_back(slot_of_site[i]);
-      ech_J.push_back(J);
-      ech_cont.push_back(cont ? 1 : 0);
-      if (cont) still.push_back(i);
-      else free_slots.push_back(slot_of_site[i]);
-    }
-    open_sites.swap(still);
-    if (last_partner[k] > k) {
-      int sl;
-      if (!free_slots.empty()) {
-        sl = free_slots.back();
-        free_slots.pop_back();
-      } else {
-        sl = nslots++;
+  auto channels = [&](bool reuse_now) {
+    ech_off.assign(L + 1, 0);
+    ech_slot.clear();
+    ech_J.clear();
+    ech_cont.clear();
+    eopen.assign(L, -1);
+    nslots = 0;
+    std::vector<int> slot_of_site(L, -1), free_slots, freed, open_sites;
+    for (int k = 0; k < L; ++k) {
+      ech_off[k] = (int)ech_slot.size();
+      std::vector<int> still;
+      freed.clear();
+      for (int i : open_sites) {
+        double J = 0.0;
+        for (int c = site_c0[i]; c < site_c0[i + 1]; ++c)
+          if (cp_j[c] == k) J += cfg->cJ[c];
+        const bool cont = last_partner[i] > k;
+        ech_slot.push_back(slot_of_site[i]);
+        ech_J.push_back(J);
+        ech_cont.push_back(cont ? 1 : 0);
+        if (cont) still.push_back(i);
+        else (reuse_now ? free_slots : freed).push_back(slot_of_site[i]);
       }
-      slot_of_site[k] = sl;
-      eopen[k] = sl;
-      open_sites.push_back(k);
+      open_sites.swap(still);
+      if (last_partner[k] > k) {
+        int sl;
+        if (!free_slots.empty()) {
+          sl = free_slots.back();
+          free_slots.pop_back();
+        } else {
+          sl = nslots++;
+        }
+        slot_of_site[k] = sl;
+        eopen[k] = sl;
+        open_sites.push_back(k);
+      }
+      free_slots.insert(free_slots.end(), freed.begin(), freed.end());
     }
-  }
-  ech_off[L] = (int)ech_slot.size();
-  if (ech_slot.empty()) {  // keep the device arrays non-empty
-    ech_slot.push_back(0);
-    ech_J.push_back(0.0);
-    ech_cont.push_back(0);
-  }
+    ech_off[L] = (int)ech_slot.size();
+    if (ech_slot.empty()) {  // keep the device arrays non-empty
+      ech_slot.push_back(0);
+      ech_J.push_back(0.0);
+      ech_cont.push_back(0);
+    }
+  };
+  channels(true);
+  const std::vector<int> tc_slot = ech_slot, tc_open = eopen;
+  const int tc_nslots = nslots;
+  channels(false);
 
   std::vector<int> h_ci(cfg->ci, cfg->ci + cfg->nC), h_cj(cfg->cj, cfg->cj + cfg->nC);
   // Terms of the MPO-term projector, in the order HeisenbergMPO::findNonZeroContributions lists
@@ -575,11 +661,11 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
   c->h_cj = h_cj;
   c->h_cq = cp_q;
   c->h_ech_off = ech_off;
-  c->h_ech_slot = ech_slot;
+  c->h_ech_slot = tc_slot;
   c->h_ech_cont = ech_cont;
-  c->h_eopen = eopen;
+  c->h_eopen = tc_open;
   c->h_ech_J = ech_J;
-  c->nslots = nslots;
+  c->nslots = tc_nslots;
   c->aT.assign(cfg->trial_dims, cfg->trial_dims + L + 1);
   c->bW.assign(cfg->walker_dims, cfg->walker_dims + L + 1);
   c->toff.resize(L);
@@ -641,7 +727,9 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
   cudaDeviceProp prop;
   if (cudaGetDeviceProperties(&prop, c->device) != cudaSuccess) return bail(fail(MPSQMC_E_CUDA, "properties"));
   c->sm_count = prop.multiProcessorCount;
-  c->smem_optin = prop.sharedMemPerBlockOptin;
+  c->smem_sm = prop.sharedMemPerMultiprocessor;
+  c->total_mem = prop.totalGlobalMem;
+  c->smem_optin = prop.sharedMemPerBlockOptin - mq::kOpBytes;  // the kernels' static part
   if (c->maxB > mq::kThreads / 2)
     return bail(fail(MPSQMC_E_UNSUPPORTED, "walker bond dimension above 128 (one QR column group per warp)"));
   {
@@ -958,7 +1046,8 @@ int mpsqmc_energy(mpsqmc_ctx *c, double *E_P) {
   mq::Dev p = make_dev(c);
   CK(cudaMemsetAsync(c->d_ctr, 0, sizeof(int) * mq::kNumCtr, c->stream));
   if (general_sweep(c))
-    mq::energy_general_kernel<<<grid_for(c, c->n_cur), mq::kThreads, c->smem_bytes, c->stream>>>(p);
+    mq::energy_general_kernel<<<std::max(1, std::min(c->n_cur, c->max_ctas_free)), c->free_threads, c->smem_bytes_free,
+                                c->stream>>>(p);
   else
     mq::energy_kernel<<<grid_for(c, c->n_cur), mq::kThreads, c->smem_bytes, c->stream>>>(p);
   CK(cudaGetLastError());
@@ -1086,7 +1175,7 @@ static int enqueue_legacy_step(mpsqmc_ctx *c, int *launches) {
   mq::Dev ps = p;
   ps.sel = c->d_changed;
   mq::set_overlap_kernel<<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(ps);
-  mq::energy_general_kernel<<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
+  mq::energy_general_kernel<<<c->max_ctas_free, c->free_threads, c->smem_bytes_free, c->stream>>>(p);
   mq::stats_kernel<<<1, 1024, 0, c->stream>>>(p, c->d_sd, c->Ndesired, c->dtau, 1, c->d_flag_pos, c->d_sw, 1,
                                               mq::kResampleLegacy);
   mq::mt_generate_kernel<<<1, 1024, 0, c->stream>>>(c->d_mt, &c->d_sd->n_flag, 0, 1, c->d_ubr);
@@ -1227,12 +1316,14 @@ static int enqueue_propagation(mpsqmc_ctx *c, int *launches, bool canon) {
       else mq::walker_step_mixed_kernel<3, false><<<g, mq::kThreads, sm, c->stream>>>(p);
     }
   } else if (gen) {
-    const size_t sm = qr_free(c) ? c->smem_bytes_noqr : c->smem_bytes;
-    if (!c->nn) mq::walker_step_general_kernel<false, 0><<<grid, mq::kThreads, sm, c->stream>>>(p);
-    else if (qr_free(c) && !c->trace_on)
-      mq::walker_step_general_kernel<true, 1, false><<<grid, mq::kThreads, sm, c->stream>>>(p);
-    else if (qr_free(c)) mq::walker_step_general_kernel<true, 1><<<grid, mq::kThreads, sm, c->stream>>>(p);
-    else mq::walker_step_general_kernel<true, 2><<<grid, mq::kThreads, sm, c->stream>>>(p);
+    if (qr_free(c) && !c->trace_on && !mlp_on(c)) {
+      const int g = c->max_ctas_free, th = c->free_threads;
+      if (c->nn) mq::walker_step_kernel_fp64<true><<<g, th, c->smem_bytes_free, c->stream>>>(p);
+      else mq::walker_step_kernel_fp64<false><<<g, th, c->smem_bytes_free, c->stream>>>(p);
+    } else {
+      if (c->nn) mq::walker_step_general_kernel<true><<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
+      else mq::walker_step_general_kernel<false><<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
+    }
   } else
     mq::walker_step_kernel<<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
   CK(cudaEventRecordWithFlags(c->ev[1], c->stream, evflags));
@@ -1242,7 +1333,7 @@ static int enqueue_propagation(mpsqmc_ctx *c, int *launches, bool canon) {
     mq::onesite_kernel<<<grid, 256, 0, c->stream>>>(p);
     mq::set_overlap_kernel<<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
     if (gen)
-      mq::energy_general_kernel<<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
+      mq::energy_general_kernel<<<c->max_ctas_free, c->free_threads, c->smem_bytes_free, c->stream>>>(p);
     else
       mq::energy_kernel<<<grid, mq::kThreads, c->smem_bytes, c->stream>>>(p);
     n += 3;

@@ -5,10 +5,8 @@
 // returns without a trailing barrier unless stated; callers place __syncthreads() between
 // dependent calls.
 //
-// FP64 products use the tensor-core DMMA instruction mma.sync.m8n8k4.f64 (tcgen05 has no f64
-// kind, so this is Blackwell's FP64 tensor path).  Fragment layouts follow the PTX ISA for
-// .f64 m8n8k4: A (8x4, row): lane holds A[lane>>2][lane&3]; B (4x8, col): B[lane&3][lane>>2];
-// C/D (8x8): C[lane>>2][2*(lane&3) + i], i = 0,1.
+// FP64 products use the tensor-core DMMA instructions (mma.sync .f64; tcgen05 has no f64 kind, so
+// this is Blackwell's FP64 tensor path).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,7 +16,65 @@ namespace mq {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr int kMaxWarps = 16;  // of the QR-free FP64 sweep (any power of two of threads up to 512)
 
+// Operand of a grouped product: element (x, k) of group g and K block kb at
+// p[x*ix + k*ik + g*sg + kb*sk] (x: a row of the left, a column of the right factor).
+template <typename T>
+struct Mat {
+  const T *p;
+  int ix, ik;
+  long sg, sk;
+};
+template <typename T, bool K>
+struct MatK : Mat<T> {};  // K: k contiguous (ik == 1)
+template <typename T>
+__device__ __forceinline__ MatK<T, false> cols(const T *p, int ld, long sg = 0, long sk = 0) {  // [x + ld k]
+  return {{p, 1, ld, sg, sk}};
+}
+template <typename T>
+__device__ __forceinline__ MatK<T, true> rows(const T *p, int ld, long sg = 0, long sk = 0) {  // [k + ld x]
+  return {{p, ld, 1, sg, sk}};
+}
+
+// A grouped product as the CTA's warps read it: each warp keeps its own copy in shared memory.  As
+// function arguments the thirty words would live in registers beside the fragments and be spilled;
+// from here a warp takes them when it sets up a tile.
+struct alignas(16) GemmOp {
+  const double *a, *b;
+  double *c;
+  int M, N, K, GM, GN, GK;
+  int aix, aik, bix, bik;
+  int ldc, ca, cb, beta;
+  long asg, ask, bsg, bsk;
+};
+__device__ __forceinline__ GemmOp *warp_op() {
+  __shared__ GemmOp ops[kMaxWarps];
+  return ops + (threadIdx.x >> 5);
+}
+constexpr int kOpBytes = kMaxWarps * sizeof(GemmOp);  // static shared memory of every kernel with products
+template <bool KA, bool KB>
+__device__ __forceinline__ void set_op(int M, int N, int K, const MatK<double, KA> &A, int GM, const MatK<double, KB> &B,
+                                       int GN, int GK, bool beta, double *C, int ldc, int ca, int cb) {
+  __syncwarp();
+  *warp_op() = GemmOp{A.p, B.p, C,  M,   N,  K,  GM,   GN,   GK,   A.ix, A.ik,
+                       B.ix, B.ik, ldc, ca, cb, beta, A.sg, A.sk, B.sg, B.sk};
+  __syncwarp();
+}
+
+// Quotient and remainder of a by b where the quotient is small, by subtraction (an integer division
+// costs more than the few rounds).
+__device__ __forceinline__ int take_out(int &a, int b) {
+  int q = 0;
+#pragma unroll 1
+  while (a >= b) {
+    a -= b;
+    ++q;
+  }
+  return q;
+}
+// mma.sync m8n8k4 .f64.  Fragments (PTX ISA), g = lane >> 2, t = lane & 3: A[g][t], B[t][g],
+// D[g][2t], D[g][2t + 1].
 __device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double b) {
   asm volatile(
       "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -26,267 +82,359 @@ __device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double
       : "d"(a), "d"(b));
 }
 
-// Check-free path for M, N, K multiples of 16: each warp computes 16x16 blocks; the K loop runs
-// in chunks of four k-steps whose 16 fragment loads are issued one chunk ahead of the DMMAs.
-template <bool TA, bool TB>
-static __device__ __forceinline__ void gemm16(int M, int N, int K, double alpha, const double *A, int lda,
-                                              const double *B, int ldb, double beta, double *C, int ldc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int bm = M >> 4, bn = N >> 4;
-  const long sa = TA ? 4 : 4L * lda, sb = TB ? 4L * ldb : 4;
-  for (int blk = warp; blk < bm * bn; blk += kWarps) {
-    const int m0 = (blk % bm) << 4, n0 = (blk / bm) << 4;
-    const int ma = m0 + g, mb = m0 + 8 + g, na = n0 + g, nb = n0 + 8 + g;
-    const double *pa0 = TA ? A + (long)lda * ma + t : A + ma + (long)lda * t;
-    const double *pa1 = TA ? A + (long)lda * mb + t : A + mb + (long)lda * t;
-    const double *pb0 = TB ? B + na + (long)ldb * t : B + t + (long)ldb * na;
-    const double *pb1 = TB ? B + nb + (long)ldb * t : B + t + (long)ldb * nb;
-    double acc[2][2][2] = {{{0.0, 0.0}, {0.0, 0.0}}, {{0.0, 0.0}, {0.0, 0.0}}};
-    double a0[4], a1[4], b0[4], b1[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      a0[u] = pa0[u * sa];
-      a1[u] = pa1[u * sa];
-      b0[u] = pb0[u * sb];
-      b1[u] = pb1[u * sb];
-    }
-    for (int k0 = 0; k0 < K; k0 += 16) {
-      double c0[4], c1[4], d0[4], d1[4];
-      const bool more = k0 + 16 < K;
-      const long off = (long)(k0 / 4 + 4);
-      if (more) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          c0[u] = pa0[(off + u) * sa];
-          c1[u] = pa1[(off + u) * sa];
-          d0[u] = pb0[(off + u) * sb];
-          d1[u] = pb1[(off + u) * sb];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        dmma884(acc[0][0][0], acc[0][0][1], a0[u], b0[u]);
-        dmma884(acc[0][1][0], acc[0][1][1], a0[u], b1[u]);
-        dmma884(acc[1][0][0], acc[1][0][1], a1[u], b0[u]);
-        dmma884(acc[1][1][0], acc[1][1][1], a1[u], b1[u]);
-      }
-      if (more) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          a0[u] = c0[u];
-          a1[u] = c1[u];
-          b0[u] = d0[u];
-          b1[u] = d1[u];
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          double *c = C + (m0 + 8 * i + g) + (long)ldc * (n0 + 8 * j + 2 * t + e);
-          const double v = alpha * acc[i][j][e];
-          *c = (beta == 0.0) ? v : v + beta * (*c);
-        }
+// Output tiles of a grouped FP64 product, for every (ga < GM, gb < GN):
+//   sum_{kb < GK} sum_{k < K} A(ga, kb)[m, k] B(gb, kb)[k, n],   m < M, n < N,
+// handed to epi.put(ga, gb, m, n, v, w, two): v of row m and (two) w of row m + 1.  KA, KB: k is
+// contiguous in A, in B (ik == 1).  A warp owns a tile of 16 rows (of one left group) by NP
+// 8-column pieces (16-column blocks of any right groups; one piece of 8 when NP == 1).
+//
+// What bounds it is the FP64 tensor pipe (64 FMA per clock and SM) once a warp gets by with few
+// instructions besides its DMMAs: a warp's dependent instructions issue every four to five cycles,
+// and four warps share a scheduler.  So the loads are 16 bytes wide wherever the operands are
+// aligned (V): the MMA's row, column and k slots are dealt out so that a lane's two rows (2g,
+// 2g+1), its columns in two neighbouring pieces (2g, 2g+1) or its two k (2t, 2t+1) are adjacent
+// in memory.  With leading dimensions of 4 mod 8 the k-contiguous shared-memory reads are free of
+// bank conflicts.  The left factor, which may come from L2, is loaded a chunk of eight k ahead.
+// Rows and columns beyond M, N read a valid neighbour and are not handed out; a last partial chunk
+// is read element by element, masked.
+// The tile of an element depends on M, N, GM, GN only: two calls with the same ones may
+// accumulate into the same output without a barrier.
+template <int NP, bool KA, bool KB, bool V, class Epi>
+__device__ __forceinline__ void dmma_tiles(const volatile GemmOp &op, Epi &epi) {
+  constexpr bool kPair = KA || KB;            // a lane's two k: 2t, 2t+1 (else t, t+4)
+  constexpr int kNext = kPair ? 1 : 4, kW = NP == 1 ? 8 : 16, kBlk = NP == 1 ? 1 : NP / 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int g = lane >> 2, t = lane & 3, kl = kPair ? 2 * t : t;
+  int mt, tiles, per, span;
+  {
+    const int n1 = (op.N + kW - 1) / kW, GN = op.GN;
+    mt = op.GM * ((op.M + 15) >> 4);
+    // blocks are dealt out from all right groups in a row, or (kOneGroup) group by group
+    span = Epi::kOneGroup ? n1 : GN * n1;
+    per = (span + kBlk - 1) / kBlk;
+    tiles = mt * per * (Epi::kOneGroup ? GN : 1);
   }
-}
-
-// C (M x N, ldc) = alpha * op(A) * op(B) + beta * C, op(A) M x K, op(B) K x N.
-//   ta == false: A[m + lda*k];  ta == true: A[k + lda*m]
-//   tb == false: B[k + ldb*n];  tb == true: B[n + ldb*k]
-// Each warp owns 16x16 output blocks (2x2 DMMA tiles).  When M, N and K are multiples of 16 the
-// check-free gemm16 path runs; otherwise element bounds are checked, so any M, N, K >= 0 is
-// valid.  Output element (m, n) is always written by the same thread for a given (M, N), so two
-// calls with the same M, N may accumulate into C without a barrier.
-static __device__ __noinline__ void cta_gemm(int M, int N, int K, double alpha, const double *A, int lda,
-                                      bool ta, const double *B, int ldb, bool tb, double beta,
-                                      double *C, int ldc) {
-  if (((M | N | K) & 15) == 0) {
-    if (ta) {
-      if (tb) gemm16<true, true>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-      else gemm16<true, false>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-    } else {
-      if (tb) gemm16<false, true>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-      else gemm16<false, false>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-    }
-    return;
-  }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int bm = (M + 15) >> 4, bn = (N + 15) >> 4;
-  for (int blk = warp; blk < bm * bn; blk += kWarps) {
-    const int m0 = (blk % bm) << 4, n0 = (blk / bm) << 4;
-    double acc[2][2][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-    const int ma = m0 + g, mb = m0 + 8 + g;
-    const int na = n0 + g, nb = n0 + 8 + g;
-    for (int k0 = 0; k0 < K; k0 += 4) {
-      const int k = k0 + t;
-      const bool kin = k < K;
-      double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
-      if (kin) {
-        if (ma < M) a0 = ta ? A[k + (long)lda * ma] : A[ma + (long)lda * k];
-        if (mb < M) a1 = ta ? A[k + (long)lda * mb] : A[mb + (long)lda * k];
-        if (na < N) b0 = tb ? B[na + (long)ldb * k] : B[k + (long)ldb * na];
-        if (nb < N) b1 = tb ? B[nb + (long)ldb * k] : B[k + (long)ldb * nb];
-      }
-      dmma884(acc[0][0][0], acc[0][0][1], a0, b0);
-      dmma884(acc[0][1][0], acc[0][1][1], a0, b1);
-      dmma884(acc[1][0][0], acc[1][0][1], a1, b0);
-      dmma884(acc[1][1][0], acc[1][1][1], a1, b1);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int m = m0 + 8 * i + g, n = n0 + 8 * j + 2 * t + e;
-          if (m < M && n < N) {
-            double *c = C + m + (long)ldc * n;
-            const double v = alpha * acc[i][j][e];
-            *c = (beta == 0.0) ? v : v + beta * (*c);
-          }
-        }
-  }
-}
-
-// Sixteen closures of two-site branch products, fused with the GEMM that forms them:
-//   out[k + 4 (s + 2 t)] = sum_{m < M, n < N} (A_s B_t)[m, n] P_k[m, n],   s, t in {0, 1}, k < 4,
-// A_s = A + s*sa (M x K, ld lda), B_t = B + t*sb (K x N, ld ldb), P_k = P + k*sp (ld ldp).
-// The products A_s B_t are never stored: each warp multiplies its 16x16 output blocks by the four
-// P blocks in the DMMA epilogue, and one CTA reduction writes the 16 sums to out (shared memory).
-// FAST requires M, N, K multiples of 16 (fragments loaded a chunk of four k-steps at a time);
-// otherwise every element access is bounds-checked.  red: >= 16*kWarps doubles.  Starts and ends with a
-// barrier inside the reduction.
-template <bool FAST>
-static __device__ __noinline__ void cta_closure16(int M, int N, int K, const double *A, int lda, long sa,
-                                                  const double *B, int ldb, long sb, const double *P, int ldp,
-                                                  long sp, double *red, double *out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int bm = (M + 15) >> 4, bn = (N + 15) >> 4;
-  double v[16];
-#pragma unroll
-  for (int q = 0; q < 16; ++q) v[q] = 0.0;
-  for (int blk = warp; blk < bm * bn; blk += kWarps) {
-    const int m0 = (blk % bm) << 4, n0 = (blk / bm) << 4;
-    const int ma = m0 + g, mb = m0 + 8 + g, na = n0 + g, nb = n0 + 8 + g;
+  int mi = warp, ti = 0;
 #pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-      const double *As = A + s * sa;
-      double acc[2][2][2][2], w[8];
+  for (int tile = warp; tile < tiles; tile += nw, mi += nw) {
+    const int n1 = (op.N + kW - 1) / kW;
+    ti += take_out(mi, mt);
+    int m0 = mi, pi = ti;
+    const int ga = take_out(m0, (op.M + 15) >> 4);
+    m0 = (m0 << 4) + 2 * g;
+    const int sp = Epi::kOneGroup ? take_out(pi, per) : 0;
+    const int left = span - pi * kBlk;  // blocks from the tile's first on
+    int p0 = pi * kBlk;
+    const int gb0 = Epi::kOneGroup ? sp : take_out(p0, n1);
+    double acc[NP][4];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) w[q] = 0.0;
+    for (int j = 0; j < NP; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0;
+#pragma unroll 1
+    for (int kb = 0; kb < op.GK; ++kb) {
+      const int K = op.K, full = K >> 3, aik = KA ? 1 : op.aik, bik = KB ? 1 : op.bik;
+      // row 2g and, where rows are not contiguous, 2g + 1
+      const double *pa0, *pa1;
+      {
+        const int M1 = op.M - 1, aix = op.aix;
+        const int r0 = (KA || !V) ? min(m0, M1) : min(m0, M1 & ~1);
+        pa0 = op.a + (ga * op.asg + kb * op.ask + (long)r0 * aix + kl * aik);
+        pa1 = (KA || !V) ? pa0 + (long)(min(m0 + 1, M1) - r0) * aix : pa0 + kNext * aik;
+      }
+      const double *pb[NP];
+      {
+        const double *b0 = op.b + (kb * op.bsk + kl * bik);
+        const int N1 = op.N - 1, bix = op.bix;
+        const long bsg = op.bsg;
+        int gb = gb0, pc = p0;
 #pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) acc[u][i][j][0] = acc[u][i][j][1] = 0.0;
-      if (FAST) {
-        // per chunk of four k-steps: all fragment loads first, then the 32 DMMAs
-        const double *pa0 = As + ma + (long)lda * t, *pa1 = As + mb + (long)lda * t;
-        const double *pb00 = B + t + (long)ldb * na, *pb01 = B + t + (long)ldb * nb;
-        const double *pb10 = pb00 + sb, *pb11 = pb01 + sb;
-        const long sA = 4L * lda;
-        for (int k0 = 0; k0 < K; k0 += 16) {
-          const int off = k0 / 4;
-          double a0[4], a1[4], b00[4], b01[4], b10[4], b11[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            a0[u] = pa0[(off + u) * sA];
-            a1[u] = pa1[(off + u) * sA];
-            b00[u] = pb00[4 * (off + u)];
-            b01[u] = pb01[4 * (off + u)];
-            b10[u] = pb10[4 * (off + u)];
-            b11[u] = pb11[4 * (off + u)];
+        for (int j = 0; j < kBlk; ++j) {
+          const double *bg = b0 + gb * bsg;
+          if (NP == 1) {
+            pb[0] = bg + (long)min(pc * 8 + g, N1) * bix;
+          } else if (KB || !V) {
+            pb[2 * j] = bg + (long)min(pc * 16 + 2 * g, N1) * bix;
+            pb[2 * j + 1] = bg + (long)min(pc * 16 + 2 * g + 1, N1) * bix;
+          } else {  // the column pair at this lane's first and second k
+            pb[2 * j] = bg + min(pc * 16 + 2 * g, N1 & ~1);
+            pb[2 * j + 1] = pb[2 * j] + kNext * bik;
           }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            dmma884(acc[0][0][0][0], acc[0][0][0][1], a0[u], b00[u]);
-            dmma884(acc[0][0][1][0], acc[0][0][1][1], a0[u], b01[u]);
-            dmma884(acc[0][1][0][0], acc[0][1][0][1], a1[u], b00[u]);
-            dmma884(acc[0][1][1][0], acc[0][1][1][1], a1[u], b01[u]);
-            dmma884(acc[1][0][0][0], acc[1][0][0][1], a0[u], b10[u]);
-            dmma884(acc[1][0][1][0], acc[1][0][1][1], a0[u], b11[u]);
-            dmma884(acc[1][1][0][0], acc[1][1][0][1], a1[u], b10[u]);
-            dmma884(acc[1][1][1][0], acc[1][1][1][1], a1[u], b11[u]);
-          }
-        }
-      } else {
-        for (int k0 = 0; k0 < K; k0 += 4) {
-          const int k = k0 + t;
-          const bool kin = k < K;
-          double a0 = 0.0, a1 = 0.0, b[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
-          if (kin) {
-            if (ma < M) a0 = As[ma + (long)lda * k];
-            if (mb < M) a1 = As[mb + (long)lda * k];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              if (na < N) b[u][0] = B[u * sb + k + (long)ldb * na];
-              if (nb < N) b[u][1] = B[u * sb + k + (long)ldb * nb];
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            dmma884(acc[u][0][0][0], acc[u][0][0][1], a0, b[u][0]);
-            dmma884(acc[u][0][1][0], acc[u][0][1][1], a0, b[u][1]);
-            dmma884(acc[u][1][0][0], acc[u][1][0][1], a1, b[u][0]);
-            dmma884(acc[u][1][1][0], acc[u][1][1][1], a1, b[u][1]);
+          if (j + 1 < left && ++pc == n1) {
+            pc = 0;
+            ++gb;
           }
         }
       }
-      // epilogue: dot the product blocks with the four P blocks
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int m = m0 + 8 * i + g, n = n0 + 8 * j + 2 * t + e;
-            if (FAST || (m < M && n < N)) {
-              const double *pp = P + m + (long)ldp * n;
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const double pk = pp[k * sp];
-                w[k] += acc[0][i][j][e] * pk;
-                w[k + 4] += acc[1][i][j][e] * pk;
-              }
-            }
-          }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        if (s == 0) {
-          v[k] += w[k];
-          v[k + 8] += w[k + 4];
+      double a[4], an[4], b[NP][2];  // a: [row 2g, 2g+1] at the first k, then at the second
+      auto load_a = [&](double (&x)[4]) {
+        if (V) {
+          const double2 u = *reinterpret_cast<const double2 *>(pa0), v = *reinterpret_cast<const double2 *>(pa1);
+          x[0] = u.x;
+          x[3] = v.y;
+          x[KA ? 2 : 1] = u.y;
+          x[KA ? 1 : 2] = v.x;
         } else {
-          v[k + 4] += w[k];
-          v[k + 12] += w[k + 4];
+          x[0] = pa0[0];
+          x[1] = pa1[0];
+          x[2] = pa0[kNext * aik];
+          x[3] = pa1[kNext * aik];
         }
+        pa0 += 8 * aik;
+        pa1 += 8 * aik;
+      };
+      auto load_b = [&]() {
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          if (V && (KB || NP > 1)) {
+            const double2 u = *reinterpret_cast<const double2 *>(pb[j]);
+            b[KB ? j : (j & ~1)][KB ? 0 : (j & 1)] = u.x;
+            b[KB ? j : (j | 1)][KB ? 1 : (j & 1)] = u.y;
+          } else {
+            b[j][0] = pb[j][0];
+            b[j][1] = pb[j][kNext * bik];
+          }
+          pb[j] += 8 * bik;
+        }
+      };
+      const bool i0 = (full << 3) + kl < K, i1 = (full << 3) + kl + kNext < K;  // this lane's k of the last chunk
+      auto tail_a = [&](double (&x)[4]) {
+        constexpr bool pairs = V && !KA;  // pa1 is the second k of row 2g, else the first k of row 2g + 1
+        const bool odd = !pairs || m0 + 1 < op.M;
+        x[0] = i0 ? pa0[0] : 0.0;
+        x[1] = i0 && odd ? (pairs ? pa0[1] : pa1[0]) : 0.0;
+        x[2] = i1 ? (pairs ? pa1[0] : pa0[kNext * aik]) : 0.0;
+        x[3] = i1 && odd ? (pairs ? pa1[1] : pa1[kNext * aik]) : 0.0;
+      };
+      auto tail_b = [&]() {
+        constexpr bool pairs = V && !KB && NP > 1;
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          const double *q = pairs ? pb[j & ~1] + (j & 1) : pb[j];
+          b[j][0] = i0 ? q[0] : 0.0;
+          b[j][1] = i1 ? q[kNext * bik] : 0.0;
+        }
+      };
+      auto mma = [&]() {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < NP; ++j) {
+            dmma884(acc[j][0], acc[j][1], a[2 * h], b[j][h]);
+            dmma884(acc[j][2], acc[j][3], a[2 * h + 1], b[j][h]);
+          }
+      };
+      if (full > 0) load_a(a);
+#pragma unroll 1
+      for (int c = 1; c < full; ++c) {
+        load_b();
+        load_a(an);
+        mma();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) a[q] = an[q];
+      }
+      if (full > 0) {
+        load_b();
+        mma();
+      }
+      if (K & 7) {
+        tail_a(a);
+        tail_b();
+        mma();
       }
     }
+    const int M = op.M, N = op.N;
+    if (m0 < M) {
+      const bool two = m0 + 1 < M;
+      int gb = gb0, pc = p0;
+#pragma unroll
+      for (int j = 0; j < kBlk; ++j)
+        if (j < left) {
+          if (NP == 1) {
+            const int n = pc * 8 + 2 * t;
+            if (n < N) epi.put(ga, gb, m0, n, acc[0][0], acc[0][2], two);
+            if (n + 1 < N) epi.put(ga, gb, m0, n + 1, acc[0][1], acc[0][3], two);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {  // slot 2t + e of piece h: column 2 (2t + e) + h
+                const int n = pc * 16 + 4 * t + 2 * e + h;
+                if (n < N) epi.put(ga, gb, m0, n, acc[2 * j + h][e], acc[2 * j + h][2 + e], two);
+              }
+          }
+          if (++pc == n1) {
+            pc = 0;
+            ++gb;
+          }
+        }
+    }
+    if (Epi::kOneGroup) epi.done(ga, sp);
   }
+}
+
+// Pieces per tile: the wider tiles where they still give every warp one.
+__device__ __forceinline__ int tile_pieces(const volatile GemmOp &op) {
+  const int N = op.N, blocks = op.GM * ((op.M + 15) >> 4) * op.GN * ((N + 15) >> 4), nw = blockDim.x >> 5;
+  return blocks >= 2 * nw ? 4 : blocks >= nw && N > 8 ? 2 : 1;
+}
+
+// One function per tile shape: together in one body they share what can be computed in front of the
+// choice, and the registers that takes push fragments to local memory.
+template <int NP, bool KA, bool KB, bool V, class Epi>
+static __device__ __noinline__ void run_tiles(double *red) {
+  const volatile GemmOp &op = *warp_op();
+  Epi epi(op, red);
+  dmma_tiles<NP, KA, KB, V>(op, epi);
+}
+template <bool KA, bool KB, class Epi>
+__device__ __forceinline__ void dmma_groups(double *red = nullptr) {
+  const volatile GemmOp &op = *warp_op();
+  const int np = tile_pieces(op);
+  // pairs are 16-byte aligned: even strides and an even base
+  const long odd = (KA ? op.aix : op.aik) | op.asg | op.ask | (KB ? op.bix : op.bik) | op.bsg | op.bsk;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(op.a) | reinterpret_cast<uintptr_t>(op.b);
+  if (!(odd & 1) && !(at & 15)) {
+    if (np == 4) run_tiles<4, KA, KB, true, Epi>(red);
+    else if (np == 2) run_tiles<2, KA, KB, true, Epi>(red);
+    else run_tiles<1, KA, KB, true, Epi>(red);
+  } else {
+    if (np == 4) run_tiles<4, KA, KB, false, Epi>(red);
+    else if (np == 2) run_tiles<2, KA, KB, false, Epi>(red);
+    else run_tiles<1, KA, KB, false, Epi>(red);
+  }
+}
+
+struct StoreEpi {
+  static constexpr bool kOneGroup = false;
+  const volatile GemmOp &op;
+  __device__ __forceinline__ StoreEpi(const volatile GemmOp &o, double *) : op(o) {}
+  __device__ __forceinline__ void put(int ga, int gb, int m, int n, double v, double w, bool two) {
+    const int ldc = op.ldc, ca = op.ca, cb = op.cb;
+    const bool beta = op.beta, wide = ((ldc | ca | cb) & 1) == 0 && (reinterpret_cast<uintptr_t>(op.c) & 15) == 0;
+    double *c = op.c + ((long)ga * ca + (long)gb * cb + m + (long)ldc * n);
+    if (wide && two) {  // row pairs are 16-byte aligned
+      double2 x = make_double2(v, w);
+      if (beta) {
+        const double2 y = *reinterpret_cast<const double2 *>(c);
+        x.x += y.x;
+        x.y += y.y;
+      }
+      *reinterpret_cast<double2 *>(c) = x;
+    } else {
+      c[0] = beta ? v + c[0] : v;
+      if (two) c[1] = beta ? w + c[1] : w;
+    }
+  }
+  __device__ __forceinline__ void done(int, int) {}
+};
+
+// C(ga, gb)[m + ldc n] = sum_kb A(ga, kb) B(gb, kb) + (beta ? C : 0), C(ga, gb) = C + ga*ca + gb*cb, of
+// the warp's op.
+template <bool KA, bool KB>
+__device__ __forceinline__ void cta_gemm_groups() {
+  dmma_groups<KA, KB, StoreEpi>();
+}
+
+// The same product for small matrices, one output element per thread and round: a tile's set-up,
+// some 300 dependent instructions, costs more than the products of up to 8 x 8 x 8 elements do this
+// way (the bonds of the smallest walks, and the ends of every chain).
+__device__ __forceinline__ bool small_product(int M, int N, int K) { return M * N * K <= 512; }
+static __device__ __noinline__ void cta_gemm_small() {
+  const volatile GemmOp &op = *warp_op();
+  const int M = op.M, N = op.N, K = op.K, GM = op.GM, GK = op.GK, aik = op.aik, bik = op.bik;
+  const int sm = 32 - __clz(M - 1), sn = 32 - __clz(N - 1);  // (N, M == 1: no bits)
+  for (int e = threadIdx.x; e < (GM * op.GN) << (sm + sn); e += blockDim.x) {
+    const int m = e & ((1 << sm) - 1), n = (e >> sm) & ((1 << sn) - 1);
+    int ga = e >> (sm + sn);
+    const int gb = take_out(ga, GM);
+    if (m >= M || n >= N) continue;
+    const double *a = op.a + (ga * op.asg + m * op.aix), *b = op.b + (gb * op.bsg + n * op.bix);
+    double *c = op.c + (ga * op.ca + gb * op.cb + m + op.ldc * n);
+    double sum = op.beta ? *c : 0.0;
+    for (int kb = 0; kb < GK; ++kb) {
+#pragma unroll 4
+      for (int k = 0; k < K; ++k) sum += a[k * aik] * b[k * bik];
+      a += op.ask;
+      b += op.bsk;
+    }
+    *c = sum;
+  }
+}
+
+// C (M x N, ldc) = op(A) * op(B) + (beta ? C : 0), op(A) M x K, op(B) K x N; any M, N, K >= 0.
+//   ta == false: A[m + lda*k];  ta == true: A[k + lda*m]
+//   tb == false: B[k + ldb*n];  tb == true: B[n + ldb*k]  (not both)
+// Two calls with the same M, N may accumulate into C without a barrier.
+static __device__ __forceinline__ void cta_gemm(int M, int N, int K, double alpha, const double *A, int lda, bool ta,
+                                                const double *B, int ldb, bool tb, double beta, double *C, int ldc) {
+  (void)alpha;  // 1 everywhere
+  const bool add = beta != 0.0;
+  if (ta) {
+    set_op(M, N, K, rows(A, lda), 1, rows(B, ldb), 1, 1, add, C, ldc, 0, 0);
+    cta_gemm_groups<true, true>();
+  } else if (tb) {
+    set_op(M, N, K, cols(A, lda), 1, cols(B, ldb), 1, 1, add, C, ldc, 0, 0);
+    cta_gemm_groups<false, false>();
+  } else {
+    set_op(M, N, K, cols(A, lda), 1, rows(B, ldb), 1, 1, add, C, ldc, 0, 0);
+    cta_gemm_groups<false, true>();
+  }
+}
+
+// Sixteen closures of two-site branch products, fused with the products that form them:
+//   out[k + 4 (s + 2 t)] = sum_{m < M, n < N} (A_s B_t)[m, n] P_k[m, n],   s, t in {0, 1}, k < 4,
+// A_s = A + s*sa (M x K, ld lda), B_t = B + t*sb (K x N, ld ldb), P_k = P + k*sp (ld ldp).  The
+// products are never stored: a warp dots its tile with the four P tiles in the epilogue and adds
+// to its own column of red (16 doubles per warp).  Ends with a barrier.
+struct ClosureEpi {
+  static constexpr bool kOneGroup = true;
+  const volatile GemmOp &op;  // c: P, ldc: its leading dimension, ca: its block stride
+  double *red;                // of this warp
+  double w[4];
+  __device__ __forceinline__ ClosureEpi(const volatile GemmOp &o, double *r) : op(o), red(r), w{0.0, 0.0, 0.0, 0.0} {}
+  __device__ __forceinline__ void put(int, int, int m, int n, double v, double v1, bool two) {
+    const double *pp = op.c + m + (long)op.ldc * n;
+    const int sp = op.ca;
 #pragma unroll
-  for (int q = 0; q < 16; ++q)
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-  __syncthreads();
-  if (lane == 0)
+    for (int k = 0; k < 4; ++k) {
+      w[k] += v * pp[(long)k * sp];
+      if (two) w[k] += v1 * pp[(long)k * sp + 1];
+    }
+  }
+  __device__ __forceinline__ void done(int s, int t) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    __syncwarp();
 #pragma unroll
-    for (int q = 0; q < 16; ++q) red[q * kWarps + warp] = v[q];
+    for (int k = 0; k < 4; ++k) {
+      double x = w[k];
+      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if (lane == k) red[(4 * (s + 2 * t) + k) * nw] += x;
+      w[k] = 0.0;
+    }
+  }
+};
+// The warps' sums in red (16 per warp) added up.  Starts and ends with a barrier.
+__device__ __forceinline__ void add_warps(const double *red, double *out) {
+  const int nw = blockDim.x >> 5;
   __syncthreads();
   if (threadIdx.x < 16) {
     double sum = 0.0;
-    for (int w = 0; w < kWarps; ++w) sum += red[threadIdx.x * kWarps + w];
+    for (int w = 0; w < nw; ++w) sum += red[threadIdx.x * nw + w];
     out[threadIdx.x] = sum;
   }
   __syncthreads();
+}
+static __device__ __forceinline__ void cta_closure_groups(double *red) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  double *mine = red + (threadIdx.x >> 5);
+  if (lane < 16) mine[lane * nw] = 0.0;
+  __syncwarp();
+  dmma_groups<false, true, ClosureEpi>(mine);
+}
+__device__ __forceinline__ void cta_closure16(int M, int N, int K, const double *A, int lda, int sa, const double *B,
+                                              int ldb, int sb, double *P, int ldp, int sp, double *red, double *out) {
+  set_op(M, N, K, cols(A, lda, sa), 2, rows(B, ldb, sb), 2, 1, false, P, ldp, sp, 0);
+  cta_closure_groups(red);
+  add_warps(red, out);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -345,59 +493,71 @@ __device__ __forceinline__ void mma_block16(float (&acc)[2][4], const float (&a)
   for (int j = 0; j < 2; ++j) mma_tf32(acc[j], ah[0], ah[1], ah[2], ah[3], bh[j][0], bh[j][1]);
 }
 
-// C (M x N, ldc) = alpha * op(A) * op(B) + beta * C in FP32 with TF32 tensor cores; the same
-// operand conventions, block ownership (16x16 output blocks per warp, so two calls with the same
-// M, N may accumulate without a barrier) and bounds rules as the FP64 cta_gemm.
+// The FP32 counterpart of cta_gemm_groups with TF32 tensor cores: a warp owns 16x16 output blocks;
+// K blocks are summed in order, each from its own accumulators (the roundings of separate calls
+// that accumulate into C).
 template <int NP>
-static __device__ __noinline__ void cta_gemm_tf32(int M, int N, int K, float alpha, const float *A, int lda,
-                                                  bool ta, const float *B, int ldb, bool tb, float beta,
-                                                  float *C, int ldc) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+static __device__ __noinline__ void cta_gemm_groups_tf32(int M, int N, int K, Mat<float> A, int GM, Mat<float> B,
+                                                         int GN, int GK, bool beta, float *C0, int ldc, int ca, int cb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int bm = (M + 15) >> 4, bn = (N + 15) >> 4;
+  const int bm = (M + 15) >> 4, bn = (N + 15) >> 4, mt = GM * bm, tiles = mt * GN * bn;
   const bool full = ((M | N | K) & 15) == 0;
-  const long sam = ta ? lda : 1, sak = ta ? 1 : lda;  // A(m, k) = A[m*sam + k*sak]
-  const long sbk = tb ? ldb : 1, sbn = tb ? 1 : ldb;  // B(k, n) = B[k*sbk + n*sbn]
-  for (int blk = warp; blk < bm * bn; blk += kWarps) {
-    const int m0 = (blk % bm) << 4, n0 = (blk / bm) << 4;
+  const int sam = A.ix, sak = A.ik, sbk = B.ik, sbn = B.ix;
+  for (int blk = warp; blk < tiles; blk += nw) {
+    const int mi = blk % mt, ni = blk / mt, ga = mi / bm, gb = ni / bn;
+    const int m0 = (mi - ga * bm) << 4, n0 = (ni - gb * bn) << 4;
     const int ma = m0 + g, mb = m0 + 8 + g;
-    float acc[2][4];
+    const float *Ab = A.p + (long)ga * A.sg, *Bb = B.p + (long)gb * B.sg;
+    float *C = C0 + ((long)ga * ca + (long)gb * cb);
+    float sum[2][4];
+    for (int kb = 0; kb < GK; ++kb, Ab += A.sk, Bb += B.sk) {
+      float acc[2][4];
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
-    if (full) {
-      const float *pa = A + ma * sam + t * sak, *pb = B + t * sbk + (n0 + g) * sbn;
-      const long a8 = 8 * sam, k4a = 4 * sak, k4b = 4 * sbk, n8 = 8 * sbn;
+        for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
+      if (full) {
+        const float *pa = Ab + ma * sam + t * sak, *pb = Bb + t * sbk + (n0 + g) * sbn;
+        const int a8 = 8 * sam, k4a = 4 * sak, k4b = 4 * sbk, n8 = 8 * sbn;
 #pragma unroll 2
-      for (int k0 = 0; k0 < K; k0 += 8) {
-        const float *qa = pa + k0 * sak, *qb = pb + k0 * sbk;
-        const float a[4] = {qa[0], qa[a8], qa[k4a], qa[a8 + k4a]};
-        const float b[2][2] = {{qb[0], qb[k4b]}, {qb[n8], qb[n8 + k4b]}};
-        mma_block16<NP>(acc, a, b);
-      }
-    } else {
-      for (int k0 = 0; k0 < K; k0 += 8) {
-        const int ka = k0 + t, kb = k0 + t + 4;
-        float a[4] = {0.f, 0.f, 0.f, 0.f}, b[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-        if (ka < K) {
-          if (ma < M) a[0] = A[ma * sam + ka * sak];
-          if (mb < M) a[1] = A[mb * sam + ka * sak];
+        for (int k0 = 0; k0 < K; k0 += 8) {
+          const float *qa = pa + k0 * sak, *qb = pb + k0 * sbk;
+          const float a[4] = {qa[0], qa[a8], qa[k4a], qa[a8 + k4a]};
+          const float b[2][2] = {{qb[0], qb[k4b]}, {qb[n8], qb[n8 + k4b]}};
+          mma_block16<NP>(acc, a, b);
         }
-        if (kb < K) {
-          if (ma < M) a[2] = A[ma * sam + kb * sak];
-          if (mb < M) a[3] = A[mb * sam + kb * sak];
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int n = n0 + 8 * j + g;
-          if (n < N) {
-            if (ka < K) b[j][0] = B[ka * sbk + n * sbn];
-            if (kb < K) b[j][1] = B[kb * sbk + n * sbn];
+      } else {
+        for (int k0 = 0; k0 < K; k0 += 8) {
+          const int ka = k0 + t, kq = k0 + t + 4;
+          float a[4] = {0.f, 0.f, 0.f, 0.f}, b[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+          if (ka < K) {
+            if (ma < M) a[0] = Ab[ma * sam + ka * sak];
+            if (mb < M) a[1] = Ab[mb * sam + ka * sak];
           }
+          if (kq < K) {
+            if (ma < M) a[2] = Ab[ma * sam + kq * sak];
+            if (mb < M) a[3] = Ab[mb * sam + kq * sak];
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int n = n0 + 8 * j + g;
+            if (n < N) {
+              if (ka < K) b[j][0] = Bb[ka * sbk + n * sbn];
+              if (kq < K) b[j][1] = Bb[kq * sbk + n * sbn];
+            }
+          }
+          mma_block16<NP>(acc, a, b);
         }
-        mma_block16<NP>(acc, a, b);
       }
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int m = (q < 2) ? ma : mb, n = n0 + 8 * j + 2 * t + (q & 1);
+          if (kb > 0) sum[j][q] = acc[j][q] + sum[j][q];
+          else sum[j][q] = beta && (full || (m < M && n < N)) ? acc[j][q] + C[m + (long)ldc * n] : acc[j][q];
+        }
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j)
@@ -405,9 +565,7 @@ static __device__ __noinline__ void cta_gemm_tf32(int M, int N, int K, float alp
       for (int q = 0; q < 4; ++q) {
         const int m = (q < 2) ? ma : mb, n = n0 + 8 * j + 2 * t + (q & 1);
         if (full || (m < M && n < N)) {
-          float *c = C + m + (long)ldc * n;
-          const float v = alpha * acc[j][q];
-          *c = (beta == 0.f) ? v : v + beta * (*c);
+          C[m + (long)ldc * n] = sum[j][q];
         }
       }
   }
@@ -508,45 +666,47 @@ static __device__ __noinline__ void cta_closure16_tf32(int M, int N, int K, cons
 }
 
 // Overloads that let the sweep be written once for FP64 (DMMA) and FP32 (TF32) work buffers.
-template <int NP>
-__device__ __forceinline__ void gemm_t(int M, int N, int K, double alpha, const double *A, int lda, bool ta,
-                                       const double *B, int ldb, bool tb, double beta, double *C, int ldc) {
-  cta_gemm(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc);
+template <int NP, bool KA, bool KB>
+__device__ __forceinline__ void gemm_g(int M, int N, int K, const MatK<double, KA> &A, int GM, const MatK<double, KB> &B,
+                                       int GN, int GK, bool beta, double *C, int ldc, long ca = 0, long cb = 0) {
+  set_op(M, N, K, A, GM, B, GN, GK, beta, C, ldc, (int)ca, (int)cb);
+  if (small_product(M, N, K)) cta_gemm_small();
+  else cta_gemm_groups<KA, KB>();
 }
-template <int NP>
-__device__ __forceinline__ void gemm_t(int M, int N, int K, float alpha, const float *A, int lda, bool ta,
-                                       const float *B, int ldb, bool tb, float beta, float *C, int ldc) {
-  cta_gemm_tf32<NP>(M, N, K, alpha, A, lda, ta, B, ldb, tb, beta, C, ldc);
+template <int NP, bool KA, bool KB>
+__device__ __forceinline__ void gemm_g(int M, int N, int K, const MatK<float, KA> &A, int GM, const MatK<float, KB> &B,
+                                       int GN, int GK, bool beta, float *C, int ldc, long ca = 0, long cb = 0) {
+  cta_gemm_groups_tf32<NP>(M, N, K, A, GM, B, GN, GK, beta, C, ldc, (int)ca, (int)cb);
 }
 
-// Sum of v over the CTA; result returned to every thread.  red: >= kWarps doubles of smem.
+// Sum of v over the CTA; result returned to every thread.  red: >= one double per warp of smem.
 __device__ __forceinline__ double cta_sum(double v, double *red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
   if (lane == 0) red[warp] = v;
   __syncthreads();
   double s = 0.0;
-#pragma unroll
-  for (int w = 0; w < kWarps; ++w) s += red[w];
+#pragma unroll 8
+  for (int w = 0; w < nw; ++w) s += red[w];
   return s;
 }
 
-// Four sums at once (one pair of barriers).  red: >= 4*kWarps doubles.
+// Four sums at once (one pair of barriers).  red: >= four doubles per warp.
 __device__ __forceinline__ void cta_sum4(double v[4], double *red) {
 #pragma unroll
   for (int q = 0; q < 4; ++q)
     for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
   if (lane == 0)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) red[q * kWarps + warp] = v[q];
+    for (int q = 0; q < 4; ++q) red[q * nw + warp] = v[q];
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     double s = 0.0;
-    for (int w = 0; w < kWarps; ++w) s += red[q * kWarps + w];
+    for (int w = 0; w < nw; ++w) s += red[q * nw + w];
     v[q] = s;
   }
 }

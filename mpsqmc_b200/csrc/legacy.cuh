@@ -50,8 +50,10 @@ __global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev p, LegacyD
     const int slot = p.slot_of[w];
     load_walker_dims(p, s, slot);
     double *W = p.walkers + (long)slot * p.wstride;
+    s.W = W;
+    s.scr = scr;
     if (tid == 0) scr[p.roff[L]] = 1.0;
-    for (int k = L - 1; k >= 1; --k) right_env_step(p, s, W, scr, k);
+    for (int k = L - 1; k >= 1; --k) right_env_step<double>(p, s, k);
     if (tid == 0) s.Lenv[0] = 1.0;
     __syncthreads();
     for (int i = 0; i < L; ++i) {
@@ -59,30 +61,19 @@ __global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev p, LegacyD
       const double *Bi = p.trial + p.toff[i];
       load_site(s.Cen, p.pb, s.sbC, W + s.woff[i], bl, br);
       __syncthreads();
-      auto left_branches = [&]() {
-        for (int tau = 0; tau < d; ++tau)
-          cta_gemm(al, br, bl, 1.0, s.Lenv, p.pa, false, s.Cen + tau * s.sbC, p.pb, false, 0.0,
-                   s.Xb + tau * s.sbX, p.pa);
-        __syncthreads();
-        for (int sg = 0; sg < d; ++sg)
-          for (int tau = 0; tau < d; ++tau)
-            cta_gemm(ar, br, al, 1.0, Bi + (long)sg * al * ar, al, true, s.Xb + tau * s.sbX, p.pa, false, 0.0,
-                     s.Pb + (sg + d * tau) * s.sbX, p.pa);
-        __syncthreads();
-      };
       for (int c = p.site_c0[i]; c < p.site_c0[i + 1]; ++c) {
         const int j = p.cp_j[c];
-        left_branches();
+        left_branches<double>(p, s, Bi, al, ar, bl, br, s.Cen, p.pb, s.sbC);
         for (int m = i + 1; m < j; ++m) {
           const int am = p.aT[m], am1 = p.aT[m + 1], bm = s.bW[m], bm1 = s.bW[m + 1];
           load_site(s.Nxt, p.pb, s.sbC, W + s.woff[m], bm, bm1);
           __syncthreads();
           const double *Bm = p.trial + p.toff[m];
-          for (int q = 0; q < kN2; ++q)
-            transfer_in_place(p, s, Bm, am, am1, bm, bm1, s.Nxt, p.pb, s.sbC, s.Pb + q * s.sbX, p.pa);
+          transfer_in_place<double>(p, s, rows(Bm, am, 0, (long)am * am1), am, am1, bm, bm1, s.Nxt, p.pb, s.sbC, s.Pb,
+                                    p.pa, kN2, s.sbX);
         }
         __syncthreads();
-        closures(p, s, j, W, scr);
+        closures<double>(p, s, j);
         if (tid < 3) {  // <Psi_T| A_i A_j |phi> for A = Sx, iSy, Sz
           const double *op = legacy_op(p, tid + 1);
           double v = 0.0;
@@ -93,7 +84,7 @@ __global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev p, LegacyD
         __syncthreads();
       }
       if (p.h != 0.0) {  // <Psi_T| Sz_i |phi>
-        left_branches();
+        left_branches<double>(p, s, Bi, al, ar, bl, br, s.Cen, p.pb, s.sbC);
         const double *R1 = scr + p.roff[i + 1];
         double v[4] = {0.0, 0.0, 0.0, 0.0};
         for (int q = tid; q < ar * br; q += kThreads) {
@@ -111,7 +102,8 @@ __global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev p, LegacyD
         __syncthreads();
       }
       // left environment through site i
-      if (i < L - 1) transfer_in_place(p, s, Bi, al, ar, bl, br, s.Cen, p.pb, s.sbC, s.Lenv, p.pa);
+      if (i < L - 1)
+        transfer_in_place<double>(p, s, rows(Bi, al, 0, (long)al * ar), al, ar, bl, br, s.Cen, p.pb, s.sbC, s.Lenv, p.pa);
     }
     // PDF, weight, sample (MPSQMC.cpp:336-353): one thread, the reference's order and divisions
     if (tid == 0) {

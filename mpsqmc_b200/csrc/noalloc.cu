@@ -105,11 +105,11 @@ int setup_device(int dev, DeviceSetup **out) {
     e = cudaGetDeviceProperties(&prop, dev);
     if (e != cudaSuccess) return err(MPSQMC_E_CUDA, std::string("properties: ") + cudaGetErrorString(e));
     e = cudaFuncSetAttribute(energy_noalloc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)prop.sharedMemPerBlockOptin);
+                             (int)prop.sharedMemPerBlockOptin - mq::kOpBytes);
     if (e != cudaSuccess) return err(MPSQMC_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
     st.scratch = static_cast<double *>(addr);
     st.sm_count = prop.multiProcessorCount;
-    st.smem_optin = (int)prop.sharedMemPerBlockOptin;
+    st.smem_optin = (int)prop.sharedMemPerBlockOptin - mq::kOpBytes;
     st.ready = true;
   }
   *out = &st;

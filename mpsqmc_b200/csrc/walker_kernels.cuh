@@ -24,6 +24,8 @@
 
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "cta_linalg.cuh"
 
 namespace mq {
@@ -31,6 +33,15 @@ namespace mq {
 constexpr int kMaxD = 2;  // local dimension implemented by the kernels
 constexpr int kN2 = kMaxD * kMaxD;
 constexpr int kTraceStride = kN2 * kN2 + 5;
+
+// Where the QR-free FP64 sweep keeps its matrix work buffers: bit k of `place` puts buffer k in shared
+// memory, the others live in the CTA's global scratch (the grid: where the host put it); nx blocks of
+// Xb (products held at a time).
+enum : int { kBufXb = 0, kBufNxt, kBufCen, kBufLenv, kBufNl, kBufGrid, kBufPb, kNumBuf };
+struct FreeLayout {
+  unsigned place;
+  int nx;
+};
 
 struct Dev {
   int L, d, nC, G, nJ;
@@ -82,6 +93,8 @@ struct Dev {
   const int *eopen;        // [L]: slot of the channel that site k opens, or -1
   long choff;              // energy channels inside a CTA's scratch: 2 "done" + 3 per slot
   long gwoff;              // matrix work buffers inside a CTA's scratch, or -1 (shared memory)
+  FreeLayout fl;           // work buffers of the QR-free FP64 sweep
+  long fwoff;              // its buffers outside shared memory, inside a CTA's scratch
   // QR-free general sweep: sites are stored as they leave the centre (rescaled to an isometry's Frobenius
   // norm) and a left norm environment (maxB x maxB, ld pb) inside the scratch gives the norm
   long nloff;              // its offset inside a CTA's scratch, or -1 (Householder QR per site)
@@ -112,9 +125,40 @@ struct SmemT {
   int *bW;      // bond dims of the walker being processed [L+1]
   long *woff;   // its site offsets [L]
   int *wsel;    // the walker index handed out by the work counter
-  int sbC, sbX;  // sigma-block strides of Cen/Nxt and of Xb/Pb
+  int sbC, sbX;  // sigma-block strides of Cen/Nxt and of Xb/Pb/Qt
+  int nx;        // blocks of Xb
+  // tables of the problem: Dev's, or on-chip copies (read in dependent chains in front of every
+  // product, and evicted from the L1 by the environments)
+  const double *grid, *tabU, *tabSq, *tabVT;
+  const int *aT, *bS, *site_c0, *cp_j, *cp_q, *eopen, *ech_off;  // bS: Dev::bW
+  const long *toff, *roff, *zoff;
+  // energy channels of the site being processed: those that close on it (J, slot), those that stay open
+  double *closeJ;
+  int *closeS, *contS, *nlist;  // nlist: how many of each
+  // general sweep: the walker being processed
+  double *W;          // its tensors
+  T *scr;             // the CTA's scratch
+  T *Fd, *Fdn, *Fch;  // energy channels: "done" (current, next), open sites
+  T *Nl;              // left norm environment (QR-free sweep), or nullptr
+  int w, slot;
 };
+// s.sc: what the threads of a CTA hand one another (1-7: sampling), and the walker's running numbers
+enum : int { kScOv = 8, kScWt = 9, kScNorm = 10 };
 using Smem = SmemT<double>;
+// The QR-free sweeps keep this table and the kernel's arguments in shared memory, in front of the
+// buffers: as registers of every thread, hoisted out of the loops over sites, they cost the
+// products their fragments (spilled around each call: 28 MB of local-memory traffic per walker
+// and step of the L = 64 chain).
+constexpr int kTableDoubles = 64, kArgDoubles = (sizeof(Dev) + 31) / 32 * 4;
+static_assert(sizeof(Smem) <= 8 * kTableDoubles, "buffer table");
+
+template <typename T>
+__host__ __device__ inline void set_lists(SmemT<T> &s, double *a, double *b, double *c, double *e) {
+  s.closeJ = a;
+  s.closeS = reinterpret_cast<int *>(b);
+  s.contS = reinterpret_cast<int *>(c);
+  s.nlist = reinterpret_cast<int *>(e);
+}
 
 // Work buffers of one CTA.  The small ones always live in shared memory.  The matrix buffers
 // (environments, site tensors, branches, QR panel) follow them in shared memory when they fit;
@@ -149,7 +193,7 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   take(s ? s->Cm : dummy, 16);
   take(s ? s->O1 : dummy, 4);
   take(s ? s->O2 : dummy, 4);
-  take(s ? s->pdf : dummy, G);
+  take(s ? s->pdf : dummy, (G + 31) & ~31);
   take(s ? s->sc : dummy, 16);
   {
     double *b, *o, *q, *m;
@@ -165,6 +209,14 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
     }
   }
   take(s ? s->qprop : dummy, mlp ? G : 0);
+  if (qr) {  // the engine's kernels
+    double *a, *b, *c, *e;
+    take(a, L);
+    take(b, (L + 1) / 2);
+    take(c, (L + 1) / 2);
+    take(e, 1);
+    if (s) set_lists(*s, a, b, c, e);
+  }
   take_big(s ? s->Lenv : dummy, (long)pa * maxB);
   take_big(s ? s->Cen : dummy, (long)pb * maxB * d);
   take_big(s ? s->Nxt : dummy, (long)pb * maxB * d);
@@ -182,7 +234,72 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   if (s) {
     s->sbC = pb * maxB;
     s->sbX = pa * maxB;
+    s->nx = d;
   }
+  return off;
+}
+
+// Work buffers of the QR-free FP64 sweep under layout fl: small ones and the placed matrix buffers from
+// base on, the others from big on (sizes as above; no Householder buffers, no proposal).  Returns
+// the doubles of shared memory; *big_doubles (if given) the others.
+__host__ __device__ inline long free_doubles(int L, int nC, int maxB, int G, int nJ, int pa, int pb,
+                                             const FreeLayout &fl, Smem *s, double *base, double *big, long *big_doubles = nullptr) {
+  long off = 0, boff = 0;
+  auto take = [&](long n) {
+    double *q = base + off;
+    off += (n + 3) & ~3L;
+    return q;
+  };
+  const int d = kMaxD;
+  Smem x{};
+  take(kTableDoubles + kArgDoubles);
+  x.red = take(16 * kMaxWarps);
+  x.M = take(16);
+  x.Cm = take(16);
+  x.O1 = take(4);
+  x.O2 = take(4);
+  x.pdf = take((G + 31) & ~31);
+  x.sc = take(16);
+  x.tabU = take(16L * nJ);
+  x.tabVT = take(16L * nJ);
+  x.tabSq = take(4L * nJ);
+  auto ints = [&](int n) { return reinterpret_cast<int *>(take((n + 1) / 2)); };
+  auto longs = [&](int n) { return reinterpret_cast<long *>(take(n)); };
+  x.aT = ints(L + 1);
+  x.bS = ints(L + 1);
+  x.site_c0 = ints(L + 1);
+  x.cp_j = ints(nC);
+  x.cp_q = ints(nC);
+  x.eopen = ints(L);
+  x.ech_off = ints(L + 1);
+  x.toff = longs(L);
+  x.roff = longs(L + 1);
+  x.zoff = longs(L);
+  {
+    double *a = take(L), *b = take((L + 1) / 2), *c = take((L + 1) / 2);
+    set_lists(x, a, b, c, take(1));
+  }
+  x.bW = ints(L + 1);
+  x.woff = longs(L);
+  x.wsel = reinterpret_cast<int *>(take(1));
+  x.sbC = pb * maxB;
+  x.sbX = pa * maxB;
+  x.nx = fl.nx;
+  auto place = [&](int k, long n) {
+    if (fl.place >> k & 1u) return take(n);
+    double *q = big + boff;
+    boff += (n + 3) & ~3L;
+    return q;
+  };
+  x.Xb = place(kBufXb, (long)x.sbX * fl.nx);
+  x.Nxt = place(kBufNxt, (long)x.sbC * d);
+  x.Cen = place(kBufCen, (long)x.sbC * d);
+  x.Lenv = place(kBufLenv, x.sbX);
+  x.Nl = place(kBufNl, (long)pb * maxB);
+  x.grid = place(kBufGrid, 4L * G);
+  x.Pb = place(kBufPb, (long)x.sbX * kN2);
+  if (s) *s = x;
+  if (big_doubles) *big_doubles = boff;
   return off;
 }
 
@@ -201,6 +318,7 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
     off += (n + 3) & ~3L;
   };
   const int d = kMaxD;
+  off += kTableDoubles + kArgDoubles;
   take(s ? s->red : dummy, 16 * kWarps);
   take(s ? s->tau : dummy, maxB);
   take(s ? s->wv : dummy, maxB);
@@ -208,7 +326,7 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
   take(s ? s->Cm : dummy, 16);
   take(s ? s->O1 : dummy, 4);
   take(s ? s->O2 : dummy, 4);
-  take(s ? s->pdf : dummy, G);
+  take(s ? s->pdf : dummy, (G + 31) & ~31);
   take(s ? s->sc : dummy, 16);
   {
     double *b, *o, *q, *m;
@@ -224,6 +342,14 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
     }
   }
   take(s ? s->qprop : dummy, mlp ? G : 0);
+  {
+    double *a, *b, *c, *e;
+    take(a, L);
+    take(b, (L + 1) / 2);
+    take(c, (L + 1) / 2);
+    take(e, 1);
+    if (s) set_lists(*s, a, b, c, e);
+  }
   float *fbase = reinterpret_cast<float *>(base + off);
   long soff = 0;  // floats placed in shared memory after the small buffers
   auto take_big = [&](float *&p, long n) {
@@ -247,18 +373,37 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
     s->Rf = nullptr;
     s->sbC = pb * maxB;
     s->sbX = pa * maxB;
+    s->nx = d;
   }
   if (big_floats) *big_floats = boff;
   return (long)sizeof(double) * off + (long)sizeof(float) * soff;
 }
 
+template <typename T>
+__device__ __forceinline__ void global_tables(const Dev &p, SmemT<T> &s) {
+  s.grid = p.grid;
+  s.tabU = p.tabU;
+  s.tabSq = p.tabSq;
+  s.tabVT = p.tabVT;
+  s.aT = p.aT;
+  s.bS = p.bW;
+  s.site_c0 = p.site_c0;
+  s.cp_j = p.cp_j;
+  s.cp_q = p.cp_q;
+  s.eopen = p.eopen;
+  s.ech_off = p.ech_off;
+  s.toff = p.toff;
+  s.roff = p.roff;
+  s.zoff = p.zoff;
+}
+
 // Carve the work buffers of the calling CTA (shared memory, plus its global scratch when the
 // matrix buffers do not fit on chip).
-// qr: the kernel uses the Householder buffers (all but the QR-free general sweep).
-__device__ __forceinline__ void carve(const Dev &p, Smem &s, double *smem_raw, bool qr = true) {
+__device__ __forceinline__ void carve(const Dev &p, Smem &s, double *smem_raw) {
   double *big = (p.gwoff >= 0) ? p.scratch + (long)blockIdx.x * p.scr_stride + p.gwoff : nullptr;
   smem_doubles(p.L, p.maxA, p.maxB, p.G, p.pa, p.pb, p.pq, &s, smem_raw, big, nullptr,
-               p.prop_mode != 0 || p.prop_collect != 0, qr);
+               p.prop_mode != 0 || p.prop_collect != 0);
+  global_tables(p, s);
 }
 // Mixed precision: the CTA's scratch is read as floats with the same element offsets.
 __device__ __forceinline__ void carve(const Dev &p, SmemT<float> &s, double *smem_raw) {
@@ -266,13 +411,60 @@ __device__ __forceinline__ void carve(const Dev &p, SmemT<float> &s, double *sme
                               : nullptr;
   smem_bytes_f32(p.L, p.maxA, p.maxB, p.G, p.pa, p.pb, &s, smem_raw, big, nullptr,
                  p.prop_mode != 0 || p.prop_collect != 0);
+  global_tables(p, s);
+}
+
+// The QR-free sweeps: table and arguments into shared memory.  Ends with a barrier.
+template <typename T>
+__device__ __forceinline__ void carve_shared(const Dev &p, double *smem_raw) {
+  const int *src = reinterpret_cast<const int *>(&p);
+  int *dst = reinterpret_cast<int *>(smem_raw + kTableDoubles);
+  for (int q = threadIdx.x; q < (int)(sizeof(Dev) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
+  if (threadIdx.x == 0) {
+    SmemT<T> s;
+    if constexpr (std::is_same<T, double>::value) {
+      free_doubles(p.L, p.nC, p.maxB, p.G, p.nJ, p.pa, p.pb, p.fl, &s, smem_raw,
+                   p.scratch + (long)blockIdx.x * p.scr_stride + p.fwoff);
+      if (!(p.fl.place >> kBufGrid & 1u)) s.grid = p.grid;
+    } else {
+      carve(p, s, smem_raw);
+    }
+    *reinterpret_cast<SmemT<T> *>(smem_raw) = s;
+  }
+  __syncthreads();
+  if constexpr (std::is_same<T, double>::value) {
+    const Smem &s = *reinterpret_cast<Smem *>(smem_raw);
+    auto copy = [&](const auto *dst, const auto *from, int n) {
+      using V = std::remove_const_t<std::remove_reference_t<decltype(*dst)>>;
+      for (int q = threadIdx.x; q < n; q += blockDim.x) const_cast<V *>(dst)[q] = from[q];
+    };
+    const int L = p.L;
+    if (s.grid != p.grid) copy(s.grid, p.grid, 4 * p.G);
+    copy(s.tabU, p.tabU, 16 * p.nJ);
+    copy(s.tabVT, p.tabVT, 16 * p.nJ);
+    copy(s.tabSq, p.tabSq, 4 * p.nJ);
+    copy(s.aT, p.aT, L + 1);
+    copy(s.bS, p.bW, L + 1);
+    copy(s.site_c0, p.site_c0, L + 1);
+    copy(s.cp_j, p.cp_j, p.nC);
+    copy(s.cp_q, p.cp_q, p.nC);
+    copy(s.eopen, p.eopen, L);
+    copy(s.ech_off, p.ech_off, L + 1);
+    copy(s.toff, p.toff, L);
+    copy(s.roff, p.roff, L + 1);
+    copy(s.zoff, p.zoff, L);
+    __syncthreads();
+  }
+}
+__device__ __forceinline__ const Dev &shared_args(const double *smem_raw) {
+  return *reinterpret_cast<const Dev *>(smem_raw + kTableDoubles);
 }
 
 // Bond dims and site offsets of the walker in `slot` into shared memory.  Ends with a barrier.
 template <typename T>
 __device__ __forceinline__ void load_walker_dims(const Dev &p, SmemT<T> &s, int slot) {
-  for (int k = threadIdx.x; k <= p.L; k += kThreads) s.bW[k] = p.wdims[(long)slot * (p.L + 1) + k];
-  for (int k = threadIdx.x; k < p.L; k += kThreads) s.woff[k] = p.wofs[(long)slot * p.L + k];
+  for (int k = threadIdx.x; k <= p.L; k += blockDim.x) s.bW[k] = p.wdims[(long)slot * (p.L + 1) + k];
+  for (int k = threadIdx.x; k < p.L; k += blockDim.x) s.woff[k] = p.wofs[(long)slot * p.L + k];
   __syncthreads();
 }
 
@@ -289,15 +481,56 @@ __device__ __forceinline__ int next_walker(SmemT<T> &s, int *ctr) {
 
 enum : int { kCtrStep = 0, kCtrSetOverlap = 1, kCtrEnergy = 2, kCtrCompress = 3, kNumCtr = 8 };
 
+// f(r, c) for every r < rows, c < columns, over the CTA's threads, without a division: a run of
+// 2^k threads (the power of two at or above rows, at most a warp) takes a column.
+template <class F>
+__device__ __forceinline__ void for_block(int nr, int nc, F f) {
+  const int sh = nr >= 32 ? 5 : 32 - __clz(nr - 1), run = 1 << sh, step = blockDim.x >> sh;
+  for (int c = threadIdx.x >> sh; c < nc; c += step)
+    for (int r = threadIdx.x & (run - 1); r < nr; r += run) f(r, c);
+}
+
+// The same for loops that read and write memory: use(r, c, get(r, c)), with the reads of kAhead elements
+// in flight before the first is used.  (The compiler keeps a read behind the writes before it, so
+// that in for_block every element waits for memory on its own.)
+template <int kAhead = 4, class G, class U>
+__device__ __forceinline__ void for_block_ahead(int nr, int nc, G get, U use) {
+  const int sh = nr >= 32 ? 5 : 32 - __clz(nr - 1), run = 1 << sh, step = blockDim.x >> sh;
+  for (int r = threadIdx.x & (run - 1); r < nr; r += run)
+    for (int c = threadIdx.x >> sh; c < nc; c += kAhead * step) {
+      // (columns beyond the last read it again and are not used)
+      const int c1 = c + step, c2 = c1 + step, c3 = c2 + step, e = nc - 1;
+      const auto v0 = get(r, c);
+      const auto v1 = get(r, min(c1, e));
+      if constexpr (kAhead == 2) {
+        use(r, c, v0);
+        if (c1 < nc) use(r, c1, v1);
+      } else {
+        const auto v2 = get(r, min(c2, e));
+        const auto v3 = get(r, min(c3, e));
+        use(r, c, v0);
+        if (c1 < nc) use(r, c1, v1);
+        if (c2 < nc) use(r, c2, v2);
+        if (c3 < nc) use(r, c3, v3);
+      }
+    }
+}
+template <typename T, int N>
+struct Vals {
+  T x[N];
+};
+
 // dst[sigma*sb + r + ld*c] = src[r + dl*(c + dr*sigma)]   (site storage -> padded smem; an
 // FP32 destination rounds the FP64 walker)
 template <typename T>
 __device__ __forceinline__ void load_site(T *dst, int ld, int sb, const double *src, int dl, int dr) {
-  const int n = dl * dr * kMaxD;
-  for (int q = threadIdx.x; q < n; q += kThreads) {
-    const int r = q % dl, rest = q / dl, c = rest % dr, s = rest / dr;
-    dst[s * sb + r + ld * c] = T(src[q]);
-  }
+  const int blk = dl * dr;
+  for_block_ahead(
+      dl, dr, [&](int r, int c) { return Vals<double, 2>{{src[r + dl * c], src[blk + r + dl * c]}}; },
+      [&](int r, int c, const Vals<double, 2> &v) {
+        dst[r + ld * c] = T(v.x[0]);
+        dst[sb + r + ld * c] = T(v.x[1]);
+      });
 }
 // Hint the L2 to fetch the n elements at p (global memory) ahead of their use: one prefetch per
 // 128-byte line, spread over the CTA's threads.  Nothing waits for it.
@@ -305,16 +538,16 @@ template <typename T>
 __device__ __forceinline__ void prefetch_l2(const T *p, long n) {
   const char *b = reinterpret_cast<const char *>(p);
   const long bytes = n * (long)sizeof(T);
-  for (long o = 128L * threadIdx.x; o < bytes; o += 128L * kThreads)
+  for (long o = 128L * threadIdx.x; o < bytes; o += 128L * blockDim.x)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(b + o));
 }
 template <typename T>
 __device__ __forceinline__ void store_site(double *dst, const T *src, int ld, int sb, int dl, int dr) {
-  const int n = dl * dr * kMaxD;
-  for (int q = threadIdx.x; q < n; q += kThreads) {
-    const int r = q % dl, rest = q / dl, c = rest % dr, s = rest / dr;
-    dst[q] = double(src[s * sb + r + ld * c]);
-  }
+  const int blk = dl * dr;
+  for_block(dl, dr, [&](int r, int c) {
+    dst[r + dl * c] = double(src[r + ld * c]);
+    dst[blk + r + dl * c] = double(src[sb + r + ld * c]);
+  });
 }
 
 // Compact-MPO / overlap environment update through one site (all threads; ends with barrier).
