@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace mq {
 
 constexpr int kThreads = 256;
@@ -40,24 +42,27 @@ __device__ __forceinline__ MatK<T, true> rows(const T *p, int ld, long sg = 0, l
 // A grouped product as the CTA's warps read it: each warp keeps its own copy in shared memory.  As
 // function arguments the thirty words would live in registers beside the fragments and be spilled;
 // from here a warp takes them when it sets up a tile.
-struct alignas(16) GemmOp {
-  const double *a, *b;
-  double *c;
+template <typename T>
+struct alignas(16) GemmOpT {
+  const T *a, *b;
+  T *c;
   int M, N, K, GM, GN, GK;
   int aix, aik, bix, bik;
   int ldc, ca, cb, beta;
   long asg, ask, bsg, bsk;
 };
-__device__ __forceinline__ GemmOp *warp_op() {
-  __shared__ GemmOp ops[kMaxWarps];
+using GemmOp = GemmOpT<double>;
+template <typename T = double>
+__device__ __forceinline__ GemmOpT<T> *warp_op() {
+  __shared__ GemmOpT<T> ops[kMaxWarps];
   return ops + (threadIdx.x >> 5);
 }
 constexpr int kOpBytes = kMaxWarps * sizeof(GemmOp);  // static shared memory of every kernel with products
-template <bool KA, bool KB>
-__device__ __forceinline__ void set_op(int M, int N, int K, const MatK<double, KA> &A, int GM, const MatK<double, KB> &B,
-                                       int GN, int GK, bool beta, double *C, int ldc, int ca, int cb) {
+template <typename T, bool KA, bool KB>
+__device__ __forceinline__ void set_op(int M, int N, int K, const MatK<T, KA> &A, int GM, const MatK<T, KB> &B,
+                                       int GN, int GK, bool beta, T *C, int ldc, int ca, int cb) {
   __syncwarp();
-  *warp_op() = GemmOp{A.p, B.p, C,  M,   N,  K,  GM,   GN,   GK,   A.ix, A.ik,
+  *warp_op<T>() = GemmOpT<T>{A.p, B.p, C,  M,   N,  K,  GM,   GN,   GK,   A.ix, A.ik,
                        B.ix, B.ik, ldc, ca, cb, beta, A.sg, A.sk, B.sg, B.sk};
   __syncwarp();
 }
@@ -261,6 +266,7 @@ __device__ __forceinline__ void dmma_tiles(const volatile GemmOp &op, Epi &epi) 
                 if (n < N) epi.put(ga, gb, m0, n, acc[2 * j + h][e], acc[2 * j + h][2 + e], two);
               }
           }
+          epi.block();
           if (++pc == n1) {
             pc = 0;
             ++gb;
@@ -272,7 +278,8 @@ __device__ __forceinline__ void dmma_tiles(const volatile GemmOp &op, Epi &epi) 
 }
 
 // Pieces per tile: the wider tiles where they still give every warp one.
-__device__ __forceinline__ int tile_pieces(const volatile GemmOp &op) {
+template <typename T>
+__device__ __forceinline__ int tile_pieces(const volatile GemmOpT<T> &op) {
   const int N = op.N, blocks = op.GM * ((op.M + 15) >> 4) * op.GN * ((N + 15) >> 4), nw = blockDim.x >> 5;
   return blocks >= 2 * nw ? 4 : blocks >= nw && N > 8 ? 2 : 1;
 }
@@ -303,27 +310,34 @@ __device__ __forceinline__ void dmma_groups(double *red = nullptr) {
   }
 }
 
+template <typename T>
+struct alignas(2 * sizeof(T)) Pair {
+  T x, y;
+};
+template <typename T>
 struct StoreEpi {
   static constexpr bool kOneGroup = false;
-  const volatile GemmOp &op;
-  __device__ __forceinline__ StoreEpi(const volatile GemmOp &o, double *) : op(o) {}
-  __device__ __forceinline__ void put(int ga, int gb, int m, int n, double v, double w, bool two) {
+  const volatile GemmOpT<T> &op;
+  __device__ __forceinline__ StoreEpi(const volatile GemmOpT<T> &o, double *) : op(o) {}
+  __device__ __forceinline__ void put(int ga, int gb, int m, int n, T v, T w, bool two) {
     const int ldc = op.ldc, ca = op.ca, cb = op.cb;
-    const bool beta = op.beta, wide = ((ldc | ca | cb) & 1) == 0 && (reinterpret_cast<uintptr_t>(op.c) & 15) == 0;
-    double *c = op.c + ((long)ga * ca + (long)gb * cb + m + (long)ldc * n);
-    if (wide && two) {  // row pairs are 16-byte aligned
-      double2 x = make_double2(v, w);
+    const bool beta = op.beta,
+               wide = ((ldc | ca | cb) & 1) == 0 && (reinterpret_cast<uintptr_t>(op.c) & (2 * sizeof(T) - 1)) == 0;
+    T *c = op.c + ((long)ga * ca + (long)gb * cb + m + (long)ldc * n);
+    if (wide && two) {  // row pairs are aligned
+      Pair<T> x{v, w};
       if (beta) {
-        const double2 y = *reinterpret_cast<const double2 *>(c);
+        const Pair<T> y = *reinterpret_cast<const Pair<T> *>(c);
         x.x += y.x;
         x.y += y.y;
       }
-      *reinterpret_cast<double2 *>(c) = x;
+      *reinterpret_cast<Pair<T> *>(c) = x;
     } else {
       c[0] = beta ? v + c[0] : v;
       if (two) c[1] = beta ? w + c[1] : w;
     }
   }
+  __device__ __forceinline__ void block() {}
   __device__ __forceinline__ void done(int, int) {}
 };
 
@@ -331,15 +345,16 @@ struct StoreEpi {
 // the warp's op.
 template <bool KA, bool KB>
 __device__ __forceinline__ void cta_gemm_groups() {
-  dmma_groups<KA, KB, StoreEpi>();
+  dmma_groups<KA, KB, StoreEpi<double>>();
 }
 
 // The same product for small matrices, one output element per thread and round: a tile's set-up,
 // some 300 dependent instructions, costs more than the products of up to 8 x 8 x 8 elements do this
 // way (the bonds of the smallest walks, and the ends of every chain).
 __device__ __forceinline__ bool small_product(int M, int N, int K) { return M * N * K <= 512; }
+template <typename T>
 static __device__ __noinline__ void cta_gemm_small() {
-  const volatile GemmOp &op = *warp_op();
+  const volatile GemmOpT<T> &op = *warp_op<T>();
   const int M = op.M, N = op.N, K = op.K, GM = op.GM, GK = op.GK, aik = op.aik, bik = op.bik;
   const int sm = 32 - __clz(M - 1), sn = 32 - __clz(N - 1);  // (N, M == 1: no bits)
   for (int e = threadIdx.x; e < (GM * op.GN) << (sm + sn); e += blockDim.x) {
@@ -347,9 +362,9 @@ static __device__ __noinline__ void cta_gemm_small() {
     int ga = e >> (sm + sn);
     const int gb = take_out(ga, GM);
     if (m >= M || n >= N) continue;
-    const double *a = op.a + (ga * op.asg + m * op.aix), *b = op.b + (gb * op.bsg + n * op.bix);
-    double *c = op.c + (ga * op.ca + gb * op.cb + m + op.ldc * n);
-    double sum = op.beta ? *c : 0.0;
+    const T *a = op.a + (ga * op.asg + m * op.aix), *b = op.b + (gb * op.bsg + n * op.bix);
+    T *c = op.c + (ga * op.ca + gb * op.cb + m + op.ldc * n);
+    T sum = op.beta ? *c : T(0);
     for (int kb = 0; kb < GK; ++kb) {
 #pragma unroll 4
       for (int k = 0; k < K; ++k) sum += a[k * aik] * b[k * bik];
@@ -380,63 +395,6 @@ static __device__ __forceinline__ void cta_gemm(int M, int N, int K, double alph
   }
 }
 
-// Sixteen closures of two-site branch products, fused with the products that form them:
-//   out[k + 4 (s + 2 t)] = sum_{m < M, n < N} (A_s B_t)[m, n] P_k[m, n],   s, t in {0, 1}, k < 4,
-// A_s = A + s*sa (M x K, ld lda), B_t = B + t*sb (K x N, ld ldb), P_k = P + k*sp (ld ldp).  The
-// products are never stored: a warp dots its tile with the four P tiles in the epilogue and adds
-// to its own column of red (16 doubles per warp).  Ends with a barrier.
-struct ClosureEpi {
-  static constexpr bool kOneGroup = true;
-  const volatile GemmOp &op;  // c: P, ldc: its leading dimension, ca: its block stride
-  double *red;                // of this warp
-  double w[4];
-  __device__ __forceinline__ ClosureEpi(const volatile GemmOp &o, double *r) : op(o), red(r), w{0.0, 0.0, 0.0, 0.0} {}
-  __device__ __forceinline__ void put(int, int, int m, int n, double v, double v1, bool two) {
-    const double *pp = op.c + m + (long)op.ldc * n;
-    const int sp = op.ca;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      w[k] += v * pp[(long)k * sp];
-      if (two) w[k] += v1 * pp[(long)k * sp + 1];
-    }
-  }
-  __device__ __forceinline__ void done(int s, int t) {
-    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      double x = w[k];
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == k) red[(4 * (s + 2 * t) + k) * nw] += x;
-      w[k] = 0.0;
-    }
-  }
-};
-// The warps' sums in red (16 per warp) added up.  Starts and ends with a barrier.
-__device__ __forceinline__ void add_warps(const double *red, double *out) {
-  const int nw = blockDim.x >> 5;
-  __syncthreads();
-  if (threadIdx.x < 16) {
-    double sum = 0.0;
-    for (int w = 0; w < nw; ++w) sum += red[threadIdx.x * nw + w];
-    out[threadIdx.x] = sum;
-  }
-  __syncthreads();
-}
-static __device__ __forceinline__ void cta_closure_groups(double *red) {
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  double *mine = red + (threadIdx.x >> 5);
-  if (lane < 16) mine[lane * nw] = 0.0;
-  __syncwarp();
-  dmma_groups<false, true, ClosureEpi>(mine);
-}
-__device__ __forceinline__ void cta_closure16(int M, int N, int K, const double *A, int lda, int sa, const double *B,
-                                              int ldb, int sb, double *P, int ldp, int sp, double *red, double *out) {
-  set_op(M, N, K, cols(A, lda, sa), 2, rows(B, ldb, sb), 2, 1, false, P, ldp, sp, 0);
-  cta_closure_groups(red);
-  add_warps(red, out);
-}
-
 // ---------------------------------------------------------------------------------------------
 // FP32 storage, TF32 tensor cores (the mixed-precision sweep)
 //
@@ -457,212 +415,346 @@ __device__ __forceinline__ uint32_t tf32_bits(float x) {
 
 __device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                          uint32_t b0, uint32_t b1) {
-  asm volatile(
+  asm(
       "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
       "{%0,%1,%2,%3};\n"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// One k-step of 8 for a 16x16 output block: A fragment a[4] (FP32 values), B fragments of the
-// two 8-column halves b[2][2]; acc[j] is the 16x8 half j.
+// x = head + tail, both TF32 (NP == 1: head alone)
 template <int NP>
-__device__ __forceinline__ void mma_block16(float (&acc)[2][4], const float (&a)[4], const float (&b)[2][2]) {
-  uint32_t ah[4], bh[2][2];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) ah[q] = tf32_bits(a[q]);
-#pragma unroll
-  for (int j = 0; j < 2; ++j)
-#pragma unroll
-    for (int q = 0; q < 2; ++q) bh[j][q] = tf32_bits(b[j][q]);
-  if (NP == 3) {
-    uint32_t at[4], bt[2][2];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) at[q] = tf32_bits(a[q] - __uint_as_float(ah[q]));
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) bt[j][q] = tf32_bits(b[j][q] - __uint_as_float(bh[j][q]));
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      mma_tf32(acc[j], at[0], at[1], at[2], at[3], bh[j][0], bh[j][1]);
-      mma_tf32(acc[j], ah[0], ah[1], ah[2], ah[3], bt[j][0], bt[j][1]);
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 2; ++j) mma_tf32(acc[j], ah[0], ah[1], ah[2], ah[3], bh[j][0], bh[j][1]);
+__device__ __forceinline__ void tf32_split(float x, uint32_t &head, uint32_t &tail) {
+  head = tf32_bits(x);
+  if (NP == 3) tail = tf32_bits(x - __uint_as_float(head));
 }
 
-// The FP32 counterpart of cta_gemm_groups with TF32 tensor cores: a warp owns 16x16 output blocks;
-// K blocks are summed in order, each from its own accumulators (the roundings of separate calls
-// that accumulate into C).
-template <int NP>
-static __device__ __noinline__ void cta_gemm_groups_tf32(int M, int N, int K, Mat<float> A, int GM, Mat<float> B,
-                                                         int GN, int GK, bool beta, float *C0, int ldc, int ca, int cb) {
+// The FP32 counterpart of dmma_tiles: the same tiles (16 rows by NP 8-column pieces) and epilogues, K in
+// chunks of 16 (two MMAs deep).  A lane's four k of a chunk are 4t .. 4t + 3 and its two rows 2g, 2g + 1,
+// so that k-contiguous operands are read 16 bytes and row- or column-contiguous ones 8 bytes at a
+// time (VA, VB: where the operand's strides and base allow it; a trial of bonds that are no
+// multiples of four does not).  What bounds it is instructions: an element that is loaded is split
+// into head and tail (PASSES == 3) for every tile it is part of, so a tile is as wide as
+// leaves every warp one; the left factor, which may come from L2, is loaded a chunk ahead.
+// Each chunk is summed in accumulators of its own, the small products first, and these are then added
+// up in FP32: the tensor cores' sums truncate, and a chain over all of K costs accuracy.  Measured on
+// the L = 64 chain (D_T = 64, D_W = 32, 1,024 walkers): 25.2 ms a step with 16x16 blocks, one
+// 4-byte load per element and one chain over K, 20.7 ms with these tiles; error against 64 bits
+// 8.2e-6 before, 1.1e-5 with the long chain, 5.5e-6 as it is.
+template <int PASSES, int NP, bool KA, bool KB, bool VA, bool VB, class Epi>
+__device__ __forceinline__ void tf32_tiles(const volatile GemmOpT<float> &op, Epi &epi) {
+  constexpr int kW = NP == 1 ? 8 : 16, kBlk = NP == 1 ? 1 : NP / 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int bm = (M + 15) >> 4, bn = (N + 15) >> 4, mt = GM * bm, tiles = mt * GN * bn;
-  const bool full = ((M | N | K) & 15) == 0;
-  const int sam = A.ix, sak = A.ik, sbk = B.ik, sbn = B.ix;
-  for (int blk = warp; blk < tiles; blk += nw) {
-    const int mi = blk % mt, ni = blk / mt, ga = mi / bm, gb = ni / bn;
-    const int m0 = (mi - ga * bm) << 4, n0 = (ni - gb * bn) << 4;
-    const int ma = m0 + g, mb = m0 + 8 + g;
-    const float *Ab = A.p + (long)ga * A.sg, *Bb = B.p + (long)gb * B.sg;
-    float *C = C0 + ((long)ga * ca + (long)gb * cb);
-    float sum[2][4];
-    for (int kb = 0; kb < GK; ++kb, Ab += A.sk, Bb += B.sk) {
-      float acc[2][4];
+  const int g = lane >> 2, t = lane & 3, kl = 4 * t;
+  int mt, tiles, per, span;
+  {
+    const int n1 = (op.N + kW - 1) / kW, GN = op.GN;
+    mt = op.GM * ((op.M + 15) >> 4);
+    span = Epi::kOneGroup ? n1 : GN * n1;
+    per = (span + kBlk - 1) / kBlk;
+    tiles = mt * per * (Epi::kOneGroup ? GN : 1);
+  }
+  int mi = warp, ti = 0;
+#pragma unroll 1
+  for (int tile = warp; tile < tiles; tile += nw, mi += nw) {
+    const int n1 = (op.N + kW - 1) / kW;
+    ti += take_out(mi, mt);
+    int m0 = mi, pi = ti;
+    const int ga = take_out(m0, (op.M + 15) >> 4);
+    m0 = (m0 << 4) + 2 * g;
+    const int sp = Epi::kOneGroup ? take_out(pi, per) : 0;
+    const int left = span - pi * kBlk;  // blocks from the tile's first on
+    int p0 = pi * kBlk;
+    const int gb0 = Epi::kOneGroup ? sp : take_out(p0, n1);
+    float sum[NP][4];
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+    for (int j = 0; j < NP; ++j) sum[j][0] = sum[j][1] = sum[j][2] = sum[j][3] = 0.f;
+#pragma unroll 1
+    for (int kb = 0; kb < op.GK; ++kb) {
+      const int K = op.K, full = K >> 4, aik = KA ? 1 : op.aik, bik = KB ? 1 : op.bik;
+      const float *pa0, *pa1;  // row 2g and row 2g + 1 (pairs of rows: pa0 alone)
+      {
+        const int M1 = op.M - 1, aix = op.aix;
+        const int r0 = (KA || !VA) ? min(m0, M1) : min(m0, M1 & ~1);
+        pa0 = op.a + (ga * op.asg + kb * op.ask + (long)r0 * aix + kl * aik);
+        pa1 = pa0 + (long)(min(m0 + 1, M1) - r0) * aix;
+      }
+      const float *pb[NP];
+      {
+        const float *b0 = op.b + (kb * op.bsk + kl * bik);
+        const int N1 = op.N - 1, bix = op.bix;
+        const long bsg = op.bsg;
+        int gb = gb0, pc = p0;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) acc[j][q] = 0.f;
-      if (full) {
-        const float *pa = Ab + ma * sam + t * sak, *pb = Bb + t * sbk + (n0 + g) * sbn;
-        const int a8 = 8 * sam, k4a = 4 * sak, k4b = 4 * sbk, n8 = 8 * sbn;
-#pragma unroll 2
-        for (int k0 = 0; k0 < K; k0 += 8) {
-          const float *qa = pa + k0 * sak, *qb = pb + k0 * sbk;
-          const float a[4] = {qa[0], qa[a8], qa[k4a], qa[a8 + k4a]};
-          const float b[2][2] = {{qb[0], qb[k4b]}, {qb[n8], qb[n8 + k4b]}};
-          mma_block16<NP>(acc, a, b);
+        for (int j = 0; j < kBlk; ++j) {
+          const float *bg = b0 + gb * bsg;
+          if (NP == 1) {
+            pb[0] = bg + (long)min(pc * 8 + g, N1) * bix;
+          } else if (KB || !VB) {
+            pb[2 * j] = bg + (long)min(pc * 16 + 2 * g, N1) * bix;
+            pb[2 * j + 1] = bg + (long)min(pc * 16 + 2 * g + 1, N1) * bix;
+          } else {  // the column pair
+            pb[2 * j] = pb[2 * j + 1] = bg + min(pc * 16 + 2 * g, N1 & ~1);
+          }
+          if (j + 1 < left && ++pc == n1) {
+            pc = 0;
+            ++gb;
+          }
         }
-      } else {
-        for (int k0 = 0; k0 < K; k0 += 8) {
-          const int ka = k0 + t, kq = k0 + t + 4;
-          float a[4] = {0.f, 0.f, 0.f, 0.f}, b[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-          if (ka < K) {
-            if (ma < M) a[0] = Ab[ma * sam + ka * sak];
-            if (mb < M) a[1] = Ab[mb * sam + ka * sak];
-          }
-          if (kq < K) {
-            if (ma < M) a[2] = Ab[ma * sam + kq * sak];
-            if (mb < M) a[3] = Ab[mb * sam + kq * sak];
-          }
+      }
+      float a[4][2], an[4][2], b[NP][4];  // a[k][row], b[piece][k]
+      auto load_a = [&](float (&x)[4][2]) {
+        if constexpr (VA && KA) {
+          const float4 u = *reinterpret_cast<const float4 *>(pa0), v = *reinterpret_cast<const float4 *>(pa1);
+          x[0][0] = u.x;
+          x[1][0] = u.y;
+          x[2][0] = u.z;
+          x[3][0] = u.w;
+          x[0][1] = v.x;
+          x[1][1] = v.y;
+          x[2][1] = v.z;
+          x[3][1] = v.w;
+        } else {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const int n = n0 + 8 * j + g;
-            if (n < N) {
-              if (ka < K) b[j][0] = Bb[ka * sbk + n * sbn];
-              if (kq < K) b[j][1] = Bb[kq * sbk + n * sbn];
+          for (int k = 0; k < 4; ++k) {
+            if constexpr (VA) {
+              const float2 u = *reinterpret_cast<const float2 *>(pa0 + k * aik);
+              x[k][0] = u.x;
+              x[k][1] = u.y;
+            } else {
+              x[k][0] = pa0[k * aik];
+              x[k][1] = pa1[k * aik];
             }
           }
-          mma_block16<NP>(acc, a, b);
+        }
+        pa0 += 16 * aik;
+        pa1 += 16 * aik;
+      };
+      auto load_b = [&]() {
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          if constexpr (VB && KB) {
+            const float4 u = *reinterpret_cast<const float4 *>(pb[j]);
+            b[j][0] = u.x;
+            b[j][1] = u.y;
+            b[j][2] = u.z;
+            b[j][3] = u.w;
+          } else if constexpr (VB && NP > 1) {
+            if (!(j & 1)) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float2 u = *reinterpret_cast<const float2 *>(pb[j] + k * bik);
+                b[j][k] = u.x;
+                b[j | 1][k] = u.y;
+              }
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) b[j][k] = pb[j][k * bik];
+          }
+          pb[j] += 16 * bik;
+        }
+      };
+      const int kt = K - (full << 4) - kl;  // how many of this lane's four k the last chunk has
+      auto tail_a = [&](float (&x)[4][2]) {
+        constexpr bool pairs = VA && !KA;
+        const bool odd = !pairs || m0 + 1 < op.M;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          x[k][0] = k < kt ? pa0[k * aik] : 0.f;
+          x[k][1] = k < kt && odd ? (pairs ? pa0[k * aik + 1] : pa1[k * aik]) : 0.f;
+        }
+      };
+      auto tail_b = [&]() {
+        constexpr bool pairs = VB && !KB && NP > 1;
+#pragma unroll
+        for (int j = 0; j < NP; ++j)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) b[j][k] = k < kt ? pb[j][k * bik + (pairs ? j & 1 : 0)] : 0.f;
+      };
+      auto mma = [&]() {
+        float acc[NP][4];
+#pragma unroll
+        for (int j = 0; j < NP; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+        uint32_t ah[2][4], at[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) tf32_split<PASSES>(a[2 * h + (q >> 1)][q & 1], ah[h][q], at[h][q]);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+          uint32_t bh[4], bt[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) tf32_split<PASSES>(b[j][q], bh[q], bt[q]);
+          if (PASSES == 3) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              mma_tf32(acc[j], at[h][0], at[h][1], at[h][2], at[h][3], bh[2 * h], bh[2 * h + 1]);
+              mma_tf32(acc[j], ah[h][0], ah[h][1], ah[h][2], ah[h][3], bt[2 * h], bt[2 * h + 1]);
+            }
+          }
+#pragma unroll
+          for (int h = 0; h < 2; ++h) mma_tf32(acc[j], ah[h][0], ah[h][1], ah[h][2], ah[h][3], bh[2 * h], bh[2 * h + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < NP; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sum[j][q] += acc[j][q];
+      };
+      if (full > 0) load_a(a);
+#pragma unroll 1
+      for (int c = 1; c < full; ++c) {
+        load_b();
+        load_a(an);
+        mma();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k][0] = an[k][0];
+          a[k][1] = an[k][1];
         }
       }
+      if (full > 0) {
+        load_b();
+        mma();
+      }
+      if (K & 15) {
+        tail_a(a);
+        tail_b();
+        mma();
+      }
+    }
+    const int M = op.M, N = op.N;
+    if (m0 < M) {
+      const bool two = m0 + 1 < M;
+      int gb = gb0, pc = p0;
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < kBlk; ++j)
+        if (j < left) {
+          if (NP == 1) {
+            const int n = pc * 8 + 2 * t;
+            if (n < N) epi.put(ga, gb, m0, n, sum[0][0], sum[0][2], two);
+            if (n + 1 < N) epi.put(ga, gb, m0, n + 1, sum[0][1], sum[0][3], two);
+          } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int m = (q < 2) ? ma : mb, n = n0 + 8 * j + 2 * t + (q & 1);
-          if (kb > 0) sum[j][q] = acc[j][q] + sum[j][q];
-          else sum[j][q] = beta && (full || (m < M && n < N)) ? acc[j][q] + C[m + (long)ldc * n] : acc[j][q];
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int n = pc * 16 + 4 * t + 2 * e + h;
+                if (n < N) epi.put(ga, gb, m0, n, sum[2 * j + h][e], sum[2 * j + h][2 + e], two);
+              }
+          }
+          epi.block();
+          if (++pc == n1) {
+            pc = 0;
+            ++gb;
+          }
         }
     }
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int m = (q < 2) ? ma : mb, n = n0 + 8 * j + 2 * t + (q & 1);
-        if (full || (m < M && n < N)) {
-          C[m + (long)ldc * n] = sum[j][q];
-        }
-      }
+    if (Epi::kOneGroup) epi.done(ga, sp);
   }
 }
 
-// Sixteen closures (the FP32/TF32 counterpart of cta_closure16):
+template <int PASSES, int NP, bool KA, bool KB, bool VA, bool VB, class Epi>
+static __device__ __noinline__ void run_tf32(double *red) {
+  const volatile GemmOpT<float> &op = *warp_op<float>();
+  Epi epi(op, red);
+  tf32_tiles<PASSES, NP, KA, KB, VA, VB>(op, epi);
+}
+template <int PASSES, bool KA, bool KB, class Epi>
+__device__ __forceinline__ void tf32_groups(double *red = nullptr) {
+  const volatile GemmOpT<float> &op = *warp_op<float>();
+  const int np = tile_pieces(op);
+  // an operand's quadruples of k are 16-byte aligned, its pairs of rows or columns 8-byte aligned
+  const bool va = !(((KA ? op.aix : op.aik) | op.asg | op.ask) & 3) && !(reinterpret_cast<uintptr_t>(op.a) & 15);
+  const bool vb = !(((KB ? op.bix : op.bik) | op.bsg | op.bsk) & 3) && !(reinterpret_cast<uintptr_t>(op.b) & 15);
+  if (va && vb) {
+    if (np == 4) run_tf32<PASSES, 4, KA, KB, true, true, Epi>(red);
+    else if (np == 2) run_tf32<PASSES, 2, KA, KB, true, true, Epi>(red);
+    else run_tf32<PASSES, 1, KA, KB, true, true, Epi>(red);
+  } else if (vb) {
+    if (np == 4) run_tf32<PASSES, 4, KA, KB, false, true, Epi>(red);
+    else if (np == 2) run_tf32<PASSES, 2, KA, KB, false, true, Epi>(red);
+    else run_tf32<PASSES, 1, KA, KB, false, true, Epi>(red);
+  } else {
+    if (np == 4) run_tf32<PASSES, 4, KA, KB, false, false, Epi>(red);
+    else if (np == 2) run_tf32<PASSES, 2, KA, KB, false, false, Epi>(red);
+    else run_tf32<PASSES, 1, KA, KB, false, false, Epi>(red);
+  }
+}
+
+// Sixteen closures of two-site branch products, fused with the products that form them:
 //   out[k + 4 (s + 2 t)] = sum_{m < M, n < N} (A_s B_t)[m, n] P_k[m, n],   s, t in {0, 1}, k < 4,
-// A_s = A + s*sa (M x K, ld lda, not transposed), B_t = B + t*sb (K x N, ld ldb), P_k = P + k*sp.
-// Partial sums leave the warps in FP64.  red: >= 16*kWarps doubles.  Ends with a barrier.
-template <int NP>
-static __device__ __noinline__ void cta_closure16_tf32(int M, int N, int K, const float *A, int lda, long sa,
-                                                       const float *B, int ldb, long sb, const float *P, int ldp,
-                                                       long sp, double *red, double *out) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int g = lane >> 2, t = lane & 3;
-  const int bm = (M + 15) >> 4, bn = (N + 15) >> 4;
-  double v[16];
+// A_s = A + s*sa (M x K, ld lda), B_t = B + t*sb (K x N, ld ldb), P_k = P + k*sp (ld ldp).  The
+// products are never stored: a warp dots its tile with the four P tiles in the epilogue and adds
+// to its own column of red (16 doubles per warp).  Ends with a barrier.
+template <typename T>
+struct ClosureEpi {
+  static constexpr bool kOneGroup = true;
+  const volatile GemmOpT<T> &op;  // c: P, ldc: its leading dimension, ca: its block stride
+  double *red;                    // of this warp
+  double w[4];
+  float x[4];                     // FP32: the sums of one block, before they join w
+  __device__ __forceinline__ ClosureEpi(const volatile GemmOpT<T> &o, double *r) : op(o), red(r), w{0.0, 0.0, 0.0, 0.0}, x{0.f, 0.f, 0.f, 0.f} {}
+  __device__ __forceinline__ void put(int, int, int m, int n, T v, T v1, bool two) {
+    const T *pp = op.c + m + (long)op.ldc * n;
+    const int sp = op.ca;
 #pragma unroll
-  for (int q = 0; q < 16; ++q) v[q] = 0.0;
-  for (int blk = warp; blk < bm * bn; blk += kWarps) {
-    const int m0 = (blk % bm) << 4, n0 = (blk / bm) << 4;
-    const int ma = m0 + g, mb = m0 + 8 + g;
-#pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-      const float *As = A + s * sa;
-      float acc[2][2][4];  // [t][n half][fragment]
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[u][j][q] = 0.f;
-      for (int k0 = 0; k0 < K; k0 += 8) {
-        const int ka = k0 + t, kb = k0 + t + 4;
-        float a[4] = {0.f, 0.f, 0.f, 0.f};
-        if (ka < K) {
-          if (ma < M) a[0] = As[ma + (long)lda * ka];
-          if (mb < M) a[1] = As[mb + (long)lda * ka];
-        }
-        if (kb < K) {
-          if (ma < M) a[2] = As[ma + (long)lda * kb];
-          if (mb < M) a[3] = As[mb + (long)lda * kb];
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          float b[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const int n = n0 + 8 * j + g;
-            if (n < N) {
-              if (ka < K) b[j][0] = B[u * sb + ka + (long)ldb * n];
-              if (kb < K) b[j][1] = B[u * sb + kb + (long)ldb * n];
-            }
-          }
-          mma_block16<NP>(acc[u], a, b);
-        }
-      }
-      // epilogue: dot the product blocks with the four P blocks
-      float w[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) w[q] = 0.f;
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int m = (q < 2) ? ma : mb, n = n0 + 8 * j + 2 * t + (q & 1);
-          if (m < M && n < N) {
-            const float *pp = P + m + (long)ldp * n;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float pk = pp[k * sp];
-              w[k] += acc[0][j][q] * pk;
-              w[k + 4] += acc[1][j][q] * pk;
-            }
-          }
-        }
+    for (int k = 0; k < 4; ++k) {
+      auto &at = [&]() -> auto & {
+        if constexpr (std::is_same<T, double>::value) return w[k];
+        else return x[k];
+      }();
+      at += v * pp[(long)k * sp];
+      if (two) at += v1 * pp[(long)k * sp + 1];
+    }
+  }
+  __device__ __forceinline__ void block() {
+    if constexpr (!std::is_same<T, double>::value) {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        v[k + 4 * s] += w[k];
-        v[k + 8 + 4 * s] += w[k + 4];
+        w[k] += (double)x[k];
+        x[k] = 0.f;
       }
     }
   }
+  __device__ __forceinline__ void done(int s, int t) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    __syncwarp();
 #pragma unroll
-  for (int q = 0; q < 16; ++q)
-    for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-  __syncthreads();
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < 16; ++q) red[q * kWarps + warp] = v[q];
+    for (int k = 0; k < 4; ++k) {
+      double v = w[k];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == k) red[(4 * (s + 2 * t) + k) * nw] += v;
+      w[k] = 0.0;
+    }
+  }
+};
+// The warps' sums in red (16 per warp) added up.  Starts and ends with a barrier.
+__device__ __forceinline__ void add_warps(const double *red, double *out) {
+  const int nw = blockDim.x >> 5;
   __syncthreads();
   if (threadIdx.x < 16) {
     double sum = 0.0;
-    for (int w = 0; w < kWarps; ++w) sum += red[threadIdx.x * kWarps + w];
+    for (int w = 0; w < nw; ++w) sum += red[threadIdx.x * nw + w];
     out[threadIdx.x] = sum;
   }
   __syncthreads();
+}
+template <typename T, int NP = 0>
+static __device__ __forceinline__ void cta_closure_groups(double *red) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  double *mine = red + (threadIdx.x >> 5);
+  if (lane < 16) mine[lane * nw] = 0.0;
+  __syncwarp();
+  if constexpr (std::is_same<T, double>::value) dmma_groups<false, true, ClosureEpi<double>>(mine);
+  else tf32_groups<NP, false, true, ClosureEpi<float>>(mine);
+}
+template <int NP = 0, typename T>
+__device__ __forceinline__ void cta_closure16(int M, int N, int K, const T *A, int lda, int sa, const T *B, int ldb,
+                                              int sb, T *P, int ldp, int sp, double *red, double *out) {
+  set_op(M, N, K, cols(A, lda, sa), 2, rows(B, ldb, sb), 2, 1, false, P, ldp, sp, 0);
+  cta_closure_groups<T, NP>(red);
+  add_warps(red, out);
 }
 
 // Overloads that let the sweep be written once for FP64 (DMMA) and FP32 (TF32) work buffers.
@@ -670,13 +762,15 @@ template <int NP, bool KA, bool KB>
 __device__ __forceinline__ void gemm_g(int M, int N, int K, const MatK<double, KA> &A, int GM, const MatK<double, KB> &B,
                                        int GN, int GK, bool beta, double *C, int ldc, long ca = 0, long cb = 0) {
   set_op(M, N, K, A, GM, B, GN, GK, beta, C, ldc, (int)ca, (int)cb);
-  if (small_product(M, N, K)) cta_gemm_small();
+  if (small_product(M, N, K)) cta_gemm_small<double>();
   else cta_gemm_groups<KA, KB>();
 }
 template <int NP, bool KA, bool KB>
 __device__ __forceinline__ void gemm_g(int M, int N, int K, const MatK<float, KA> &A, int GM, const MatK<float, KB> &B,
                                        int GN, int GK, bool beta, float *C, int ldc, long ca = 0, long cb = 0) {
-  cta_gemm_groups_tf32<NP>(M, N, K, A, GM, B, GN, GK, beta, C, ldc, (int)ca, (int)cb);
+  set_op(M, N, K, A, GM, B, GN, GK, beta, C, ldc, (int)ca, (int)cb);
+  if (small_product(M, N, K)) cta_gemm_small<float>();
+  else tf32_groups<NP, KA, KB, StoreEpi<float>>();
 }
 
 // Sum of v over the CTA; result returned to every thread.  red: >= one double per warp of smem.

@@ -333,10 +333,7 @@ static __device__ __forceinline__ void closures_products(const Dev &p, SmemT<T> 
   gemm_g<NP>(a2, bj, b2, cols(Rn, a2), 1, cols(s.Nxt, p.pb, s.sbC), d, 1, false, s.Xb, p.pa, 0, s.sbX);
   __syncthreads();
   // M[k + 4 (s' + 2 t')] = <P_k, B_j[s'] Y[t']>, the products formed and dotted in one pass
-  if constexpr (std::is_same<T, double>::value)
-    cta_closure16(aj, bj, a2, Bj, aj, aj * a2, s.Xb, p.pa, s.sbX, s.Pb, p.pa, s.sbX, s.red, s.M);
-  else
-    cta_closure16_tf32<NP>(aj, bj, a2, Bj, aj, (long)aj * a2, s.Xb, p.pa, s.sbX, s.Pb, p.pa, s.sbX, s.red, s.M);
+  cta_closure16<NP>(aj, bj, a2, Bj, aj, aj * a2, s.Xb, p.pa, s.sbX, s.Pb, p.pa, s.sbX, s.red, s.M);
 }
 
 // The 16 closures of coupling (i, j), left branches in Pb: against the stored right branches of
