@@ -228,27 +228,45 @@ static __device__ __noinline__ void env_build(const Dev &p, SmemT<T> &s, int k) 
     oy[e] = T(p.opISy[e]);
     oz[e] = T(p.opSz[e]);
   }
-  for_block_ahead<4>(
-      al, bl,
-      [&](int r, int c) {
-        Vals<T, kN2> v{{Fd[r + lda * c], T(0), T(0), T(0)}};
-        for (int e = 0; e < n; ++e) {
-          const T J = T(s.closeJ[e]);
-          const T *F = Fch + 3L * s.closeS[e] * fm + (r + lda * c);
-          v.x[1] += J * F[0];
-          v.x[2] += J * F[fm];
-          v.x[3] += J * F[2 * fm];
-        }
-        return v;
-      },
-      [&](int r, int c, const Vals<T, kN2> &v) {
+  // Four columns at a time, the channels in the outer loop: a channel's twelve reads are in flight together.
+  // Element by element each read waited for the one before, 24,000 cycles at a site of the L = 64
+  // chain, an eighth of its FP64 step (1,024 walkers: 24.9 ms, now 23.8 ms; 8x8 lattice unchanged).
+  const int sh = al >= 32 ? 5 : 32 - __clz(al - 1), run = 1 << sh, step = blockDim.x >> sh;
+  for (int r = threadIdx.x & (run - 1); r < al; r += run)
+    for (int c0 = threadIdx.x >> sh; c0 < bl; c0 += 4 * step) {
+      T v[4][kN2];
+      int at[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        at[u] = r + lda * min(c0 + u * step, bl - 1);
+        v[u][0] = Fd[at[u]];
+        v[u][1] = v[u][2] = v[u][3] = T(0);
+      }
+      for (int e = 0; e < n; ++e) {
+        const T J = T(s.closeJ[e]);
+        const T *F = Fch + 3L * s.closeS[e] * fm;
+        T f[4][3];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) f[u][q] = F[q * fm + at[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) v[u][q + 1] += J * f[u][q];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int c = c0 + u * step;
+        if (c >= bl) break;
 #pragma unroll
         for (int o = 0; o < kN2; ++o) {
           const int sg = o % d, tau = o / d;
           (sg == 0 ? X : Y)[tau * sb + r + pa * c] =
-              ((sg == tau) ? v.x[0] : T(0)) + ox[o] * v.x[1] - oy[o] * v.x[2] + oz[o] * v.x[3];
+              ((sg == tau) ? v[u][0] : T(0)) + ox[o] * v[u][1] - oy[o] * v[u][2] + oz[o] * v[u][3];
         }
-      });
+      }
+    }
 }
 
 // Left environments through the final tensor Tm of site k (Tm[s] bl x br, column stride cs,
