@@ -431,7 +431,11 @@ __device__ __forceinline__ void take_point(const Dev &p, SmemT<T> &s, int jq, in
 // The CDF scan is one warp's: lane k holds the run of grid points from k*per on (stored per-major,
 // so that its reads are free of conflicts), a prefix sum over the lanes places the run, and the
 // first lane whose running sum passes u has the point (a serial scan by one thread took 7,000
-// cycles of a coupling on average).
+// cycles of a coupling on average).  The sum in front of a lane and the last running sum of the lane
+// before it are rounded differently; a uniform between the two goes to the next point of nonzero
+// probability (behind the last sum: to the last such point), as the sampled point's sum C x x has to
+// be positive.  Comparisons are those of the
+// serial scan: a NaN (the sum of the PDF is zero) ends it at the first point.
 template <typename T>
 static __device__ __noinline__ void sample_grid(const Dev &p, SmemT<T> &s, int c, int jq) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -467,14 +471,21 @@ static __device__ __noinline__ void sample_grid(const Dev &p, SmemT<T> &s, int c
     if (lane == 0) at = 0.0;
     int hit = per;
     for (int i = 0; i < per; ++i) {
-      at += s.pdf[32 * i + lane];
-      if (hit == per && at * pinv > u) hit = i;
+      const double v = s.pdf[32 * i + lane];
+      at += v;
+      const double x = at * pinv;
+      if (hit == per && !(x <= u) && (v > 0.0 || isnan(x))) hit = i;
     }
     const unsigned who = __ballot_sync(full, hit < per);
-    int count = p.G - 1;
+    int count;
     if (who) {
       const int src = __ffs(who) - 1;
-      count = min(count, src * per + __shfl_sync(full, hit, src));
+      count = min(p.G - 1, src * per + __shfl_sync(full, hit, src));
+    } else {  // u beyond the last sum by rounding: the last point of nonzero probability
+      int last = -1;
+      for (int i = 0; i < per; ++i)
+        if (s.pdf[32 * i + lane] > 0.0) last = lane * per + i;
+      count = __reduce_max_sync(full, last);
     }
     take_point(p, s, jq, count, u, pnorm);
   }
