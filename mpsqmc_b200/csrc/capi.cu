@@ -94,8 +94,8 @@ struct mpsqmc_ctx {
   std::vector<long> toff, woff, roff, nroff, zoff;
   long wsize = 0, wstride = 0, scr_stride = 0, foff = 0, gwoff = -1;
   long scr_base = 0;                    // scratch doubles per CTA before the matrix work buffers
-  long all_doubles = 0, big_doubles = 0;  // work buffers: all of them / the matrix ones
-  long mlp_doubles = 0;                 // the learned proposal's small buffers (on chip while it is in use)
+  long all_doubles = 0;                 // all work buffers
+  long lwoff = -1, lwoff_mixed = -1;    // buffers by length or grid inside a CTA's scratch, or -1 (on chip)
   size_t smem_optin = 0, smem_sm = 0, total_mem = 0;  // of the device: shared memory of a CTA, of an SM; memory
   bool global_work = false;             // matrix work buffers in global scratch
   int maxA = 1, maxB = 1, pa = 4, pb = 4, pq = 4;
@@ -266,6 +266,8 @@ mq::Dev make_dev(mpsqmc_ctx *c) {
   p.eopen = c->d_eopen;
   p.choff = c->choff;
   p.gwoff = c->gwoff;
+  p.lwoff = c->lwoff;
+  p.lwoff_mixed = c->lwoff_mixed;
   p.fl = c->fl;
   p.fwoff = c->fwoff;
   p.wdims = c->d_wdims;
@@ -414,9 +416,14 @@ void free_shape(const mpsqmc_ctx *c, int *threads, int *ctas) {
   *ctas = n;
 }
 
-// That sweep's buffers (layout_workspace's part for it).  The matrix buffers go to shared memory in the
-// order of their use as right factors of products, as far as the share of a CTA reaches (with
-// room for more products at a time where all of them fit); a CTA's global scratch holds the rest.
+// That sweep's buffers (layout_workspace's part for it).  First the small ones that every coupling or
+// site reads, then the matrix buffers in the order of their use as right factors of products, as
+// far as the share of a CTA reaches (with room for more products at a time where all of them fit);
+// a CTA's global scratch holds the rest.  The problem's tables come first while they are small
+// (kSmallTable: 64 sites take 3.0 KB, a coupling strength 288 bytes) and last, if there is room,
+// where they are not: a coupling reads a few of their words, a product reads its buffers whole.
+// The PDF and the walker's dims, written by the sweep, stay on chip while a CTA can hold them.
+constexpr size_t kSmallTable = 4096;
 int layout_free(mpsqmc_ctx *c, bool force_global) {
   int threads = 0, ctas = 0;
   free_shape(c, &threads, &ctas);
@@ -426,20 +433,27 @@ int layout_free(mpsqmc_ctx *c, bool force_global) {
     return sizeof(double) * (size_t)mq::free_doubles(c->L, c->nC, c->maxB, c->G, c->nJ, c->pa, c->pb, f, nullptr, nullptr,
                                                      nullptr, big);
   };
-  const unsigned every = (1u << mq::kNumBuf) - 1;
   mq::FreeLayout f{0u, 2};
+  auto add = [&](int k, size_t limit) {
+    const mq::FreeLayout g{f.place | 1u << k, 2};
+    if (bytes(g, nullptr) <= limit) f = g;
+  };
+  for (int k : {mq::kBufPdf, mq::kBufDims}) add(k, c->smem_optin);
+  for (int k : {mq::kBufSites, mq::kBufCoup, mq::kBufTab})
+    if (bytes({1u << k, 2}, nullptr) - bytes({0u, 2}, nullptr) <= kSmallTable) add(k, force_global ? c->smem_optin : share);
+  const mq::FreeLayout small = f;
+  const unsigned matrix = (1u << mq::kNumMat) - 1;
   for (int nx : {8, 6, 4})
-    if (!f.place && bytes({every, nx}, nullptr) <= share) f = {every, nx};
-  if (!f.place)
-    for (int k = 0; k < mq::kNumBuf; ++k) {
-      const mq::FreeLayout g{f.place | 1u << k, 2};
-      if (bytes(g, nullptr) <= share) f = g;
-    }
+    if (f.nx == 2 && bytes({small.place | matrix, nx}, nullptr) <= share) f = {small.place | matrix, nx};
+  if (f.nx == 2)
+    for (int k = 0; k < mq::kNumMat; ++k) add(k, share);
+  for (int k : {mq::kBufCoup, mq::kBufSites, mq::kBufTab}) {
+    const mq::FreeLayout g{f.place | 1u << k, f.nx};
+    if (bytes(g, nullptr) <= share) f = g;
+  }
   c->fl = f;
   long big = 0;
   c->smem_bytes_free = bytes(f, &big);
-  if (c->smem_bytes_free > c->smem_optin)
-    return fail(MPSQMC_E_UNSUPPORTED, "grid too large for the shared-memory budget of one CTA");
   c->fwoff = (c->scr_base + 31) & ~31L;
   c->scr_stride = std::max(c->scr_stride, (c->fwoff + big + 31) & ~31L);
   for (const void *k : {(const void *)mq::walker_step_kernel_fp64<true>, (const void *)mq::walker_step_kernel_fp64<false>,
@@ -457,19 +471,23 @@ int layout_free(mpsqmc_ctx *c, bool force_global) {
 
 int layout_workspace(mpsqmc_ctx *c, bool force_global) {
   const bool mlp = mlp_on(c);
-  const long all = c->all_doubles + (mlp ? c->mlp_doubles : 0);
-  const bool global = force_global || sizeof(double) * (size_t)all > c->smem_optin;
-  c->scr_stride = (c->scr_base + 31) & ~31L;
-  c->gwoff = -1;
-  c->smem_bytes = sizeof(double) * (size_t)all;
-  if (global) {
-    c->gwoff = c->scr_stride;
-    c->scr_stride = (c->gwoff + c->big_doubles + 31) & ~31L;
-    c->smem_bytes = sizeof(double) * (size_t)(all - c->big_doubles);
-  }
-  c->global_work = global;
-  if (c->smem_bytes > c->smem_optin)
+  if (sizeof(double) * (size_t)mq::limit_doubles(c->L, c->maxB, c->G, mlp) > c->smem_optin + mq::kOpBytes)
     return fail(MPSQMC_E_UNSUPPORTED, "grid too large for the shared-memory budget of one CTA");
+  double some = 0.0;  // an address: buffers outside shared memory
+  float somef = 0.f;
+  const long base = (c->scr_base + 31) & ~31L;
+  auto bytes = [&](bool big, bool lng, long *nbig, long *nlong) {
+    return sizeof(double) * (size_t)mq::smem_doubles(c->L, c->maxA, c->maxB, c->G, c->pa, c->pb, c->pq, nullptr, nullptr,
+                                                     big ? &some : nullptr, nbig, mlp, true, lng ? &some : nullptr, nlong);
+  };
+  long nbig = 0, nlong = 0;
+  const bool global = force_global || bytes(false, false, nullptr, nullptr) > c->smem_optin;
+  const bool lng = bytes(global, false, nullptr, nullptr) > c->smem_optin;
+  c->smem_bytes = bytes(global, lng, &nbig, &nlong);
+  c->gwoff = global ? base : -1;
+  c->lwoff = lng ? base + ((nbig + 31) & ~31L) : -1;
+  c->scr_stride = lng ? c->lwoff + ((nlong + 31) & ~31L) : global ? base + ((nbig + 31) & ~31L) : base;
+  c->global_work = global;
   const void *kernels[] = {(const void *)mq::walker_step_kernel, (const void *)mq::set_overlap_kernel,
                            (const void *)mq::energy_kernel, (const void *)mq::walker_step_general_kernel<true>,
                            (const void *)mq::walker_step_general_kernel<false>, (const void *)mq::legacy_step_kernel};
@@ -483,11 +501,16 @@ int layout_workspace(mpsqmc_ctx *c, bool force_global) {
     if (rc) return rc;
   }
   // mixed-precision sweep: FP32 matrix buffers next to the small FP64 ones, on chip unless the
-  // FP64 buffers were placed in global scratch
+  // FP64 buffers were placed in global scratch (whose elements are floats here)
+  auto mixed_bytes = [&](bool lng_f, long *nb, long *nl) {
+    return (size_t)mq::smem_bytes_f32(c->L, c->maxA, c->maxB, c->G, c->pa, c->pb, nullptr, nullptr, global ? &somef : nullptr,
+                                      nb, mlp, lng_f ? &some : nullptr, nl);
+  };
+  const bool lng_f = mixed_bytes(false, nullptr, nullptr) > c->smem_optin;
   long big_floats = 0;
-  const long mixed_all = mq::smem_bytes_f32(c->L, c->maxA, c->maxB, c->G, c->pa, c->pb, nullptr, nullptr, nullptr,
-                                            &big_floats, mlp);
-  c->smem_bytes_mixed = global ? (size_t)(mixed_all - (long)sizeof(float) * big_floats) : (size_t)mixed_all;
+  c->smem_bytes_mixed = mixed_bytes(lng_f, &big_floats, &nlong);
+  c->lwoff_mixed = lng_f ? base + ((big_floats + 31) & ~31L) : -1;
+  if (lng_f) c->scr_stride = std::max(c->scr_stride, c->lwoff_mixed + ((2 * nlong + 31) & ~31L));
   const void *mk[] = {(const void *)mq::walker_step_mixed_kernel<1, true>, (const void *)mq::walker_step_mixed_kernel<3, true>,
                       (const void *)mq::walker_step_mixed_kernel<1, false>, (const void *)mq::walker_step_mixed_kernel<3, false>};
   for (const void *k : mk)
@@ -684,10 +707,7 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
   c->pa = mq::padld(std::max(c->maxA, c->maxB));  // slots also hold walker-row matrices
   c->pb = mq::padld(c->maxB);
   c->pq = mq::padld(d * c->maxB);
-  c->all_doubles =
-      mq::smem_doubles(L, c->maxA, c->maxB, c->G, c->pa, c->pb, c->pq, nullptr, nullptr, nullptr, &c->big_doubles);
-  c->mlp_doubles = mq::smem_doubles(L, c->maxA, c->maxB, c->G, c->pa, c->pb, c->pq, nullptr, nullptr, nullptr,
-                                    nullptr, true) - c->all_doubles;
+  c->all_doubles = mq::smem_doubles(L, c->maxA, c->maxB, c->G, c->pa, c->pb, c->pq, nullptr, nullptr);
   c->roff.resize(L + 1);
   long ro = 0;
   for (int k = 0; k <= L; ++k) {

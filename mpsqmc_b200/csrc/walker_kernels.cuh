@@ -34,10 +34,19 @@ constexpr int kMaxD = 2;  // local dimension implemented by the kernels
 constexpr int kN2 = kMaxD * kMaxD;
 constexpr int kTraceStride = kN2 * kN2 + 5;
 
-// Where the QR-free FP64 sweep keeps its matrix work buffers: bit k of `place` puts buffer k in shared
-// memory, the others live in the CTA's global scratch (the grid: where the host put it); nx blocks of
-// Xb (products held at a time).
-enum : int { kBufXb = 0, kBufNxt, kBufCen, kBufLenv, kBufNl, kBufGrid, kBufPb, kNumBuf };
+// Where the QR-free FP64 sweep keeps its buffers: bit k of `place` puts buffer k in shared memory.  The
+// others live in the CTA's global scratch, or (the grid and the problem's tables) where the host put
+// them; nx blocks of Xb (products held at a time).  Buffers whose size a problem's length, couplings
+// or grid set are among them, so that none of these can be too large for a CTA.
+enum : int {
+  kBufXb = 0, kBufNxt, kBufCen, kBufLenv, kBufNl, kBufGrid, kBufPb, kNumMat,  // the matrix buffers and the grid
+  kBufPdf = kNumMat,  // PDF, channel lists
+  kBufDims,           // bond dims and site offsets of the walker
+  kBufSites,          // tables by site
+  kBufCoup,           // tables by coupling
+  kBufTab,            // tables by coupling strength
+  kNumBuf
+};
 struct FreeLayout {
   unsigned place;
   int nx;
@@ -93,6 +102,7 @@ struct Dev {
   const int *eopen;        // [L]: slot of the channel that site k opens, or -1
   long choff;              // energy channels inside a CTA's scratch: 2 "done" + 3 per slot
   long gwoff;              // matrix work buffers inside a CTA's scratch, or -1 (shared memory)
+  long lwoff, lwoff_mixed; // buffers by length or grid (smem_doubles, smem_bytes_f32) inside it, or -1
   FreeLayout fl;           // work buffers of the QR-free FP64 sweep
   long fwoff;              // its buffers outside shared memory, inside a CTA's scratch
   // QR-free general sweep: sites are stored as they leave the centre (rescaled to an isometry's Frobenius
@@ -152,24 +162,43 @@ using Smem = SmemT<double>;
 constexpr int kTableDoubles = 64, kArgDoubles = (sizeof(Dev) + 31) / 32 * 4;
 static_assert(sizeof(Smem) <= 8 * kTableDoubles, "buffer table");
 
+// The PDF (32 values for each grid point of a lane, sample_grid) and the lists of a site's channels share
+// their place: a site's couplings are sampled before its environments are built.
+__host__ __device__ inline long pdf_doubles(int L, int G, bool lists) {
+  const long pdf = (G + 31) & ~31, ls = lists ? ((L + 3) & ~3L) + 2 * (((L + 1) / 2 + 3) & ~3L) + 4 : 0;
+  return pdf > ls ? pdf : ls;
+}
 template <typename T>
-__host__ __device__ inline void set_lists(SmemT<T> &s, double *a, double *b, double *c, double *e) {
-  s.closeJ = a;
-  s.closeS = reinterpret_cast<int *>(b);
-  s.contS = reinterpret_cast<int *>(c);
-  s.nlist = reinterpret_cast<int *>(e);
+__host__ __device__ inline void set_pdf(SmemT<T> &s, int L, double *p, bool lists) {
+  s.pdf = p;
+  if (!lists) return;
+  const long half = ((L + 1) / 2 + 3) & ~3L;
+  s.closeJ = p;
+  p += (L + 3) & ~3L;
+  s.closeS = reinterpret_cast<int *>(p);
+  s.contS = reinterpret_cast<int *>(p + half);
+  s.nlist = reinterpret_cast<int *>(p + 2 * half);
 }
 
-// Work buffers of one CTA.  The small ones always live in shared memory.  The matrix buffers
+// What a problem's length and grid may take, in doubles: a grid or chain beyond it is refused.
+__host__ inline long limit_doubles(int L, int maxB, int G, bool mlp) {
+  auto r = [](long n) { return (n + 3) & ~3L; };
+  return 16 * kWarps + 2 * r(maxB) + 60 + r(G) + r((L + 2) / 2) + r(L) + (mlp ? 400 + r(G) : 0);
+}
+
+// Work buffers of one CTA.  The small ones live in shared memory.  The matrix buffers
 // (environments, site tensors, branches, QR panel) follow them in shared memory when they fit;
 // for large bond dimensions they live in the CTA's global scratch instead (big != nullptr), where
-// the GEMMs read them through L1/L2.  Returns the doubles placed in shared memory; *big_doubles
-// (if given) receives the size of the matrix buffers.  mlp: the learned proposal's buffers.
+// the GEMMs read them through L1/L2.  The small ones that grow with the chain or the grid go there
+// too (lng != nullptr) where they leave no room for the others.  Returns the doubles placed in
+// shared memory; *big_doubles and *lng_doubles (if given) receive the sizes of the matrix buffers
+// and of the long ones.  mlp: the learned proposal's buffers.
 __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, int pa, int pb, int pq,
                                               Smem *s, double *base, double *big = nullptr,
-                                              long *big_doubles = nullptr, bool mlp = false, bool qr = true) {
+                                              long *big_doubles = nullptr, bool mlp = false, bool qr = true,
+                                              double *lng = nullptr, long *lng_doubles = nullptr) {
   (void)maxA;  // the blocks are sized by the padded pa, pb
-  long off = 0, boff = 0;
+  long off = 0, boff = 0, loff = 0;
   double *dummy;
   auto take = [&](double *&p, long n) {
     if (s) p = base + off;
@@ -185,6 +214,12 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
     }
     boff += r;
   };
+  auto take_long = [&](long n) {
+    const long r = (n + 3) & ~3L;
+    double *p = lng ? lng + loff : base + off;
+    (lng ? loff : off) += r;
+    return p;
+  };
   const int d = kMaxD;
   take(s ? s->red : dummy, 16 * kWarps);
   take(s ? s->tau : dummy, maxB);
@@ -193,15 +228,13 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   take(s ? s->Cm : dummy, 16);
   take(s ? s->O1 : dummy, 4);
   take(s ? s->O2 : dummy, 4);
-  take(s ? s->pdf : dummy, (G + 31) & ~31);
   take(s ? s->sc : dummy, 16);
   {
-    double *b, *o, *q, *m;
-    take(b, (L + 2) / 2);
-    take(o, L);
-    take(q, 1);
-    take(m, mlp ? 400 : 0);
+    double *x = take_long(pdf_doubles(L, G, qr)), *b = take_long((L + 2) / 2), *o = take_long(L), *q = nullptr, *m = nullptr;
+    take(s ? q : dummy, 1);
+    take(s ? m : dummy, mlp ? 400 : 0);
     if (s) {
+      set_pdf(*s, L, x, qr);
       s->bW = reinterpret_cast<int *>(b);
       s->woff = reinterpret_cast<long *>(o);
       s->wsel = reinterpret_cast<int *>(q);
@@ -209,14 +242,6 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
     }
   }
   take(s ? s->qprop : dummy, mlp ? G : 0);
-  if (qr) {  // the engine's kernels
-    double *a, *b, *c, *e;
-    take(a, L);
-    take(b, (L + 1) / 2);
-    take(c, (L + 1) / 2);
-    take(e, 1);
-    if (s) set_lists(*s, a, b, c, e);
-  }
   take_big(s ? s->Lenv : dummy, (long)pa * maxB);
   take_big(s ? s->Cen : dummy, (long)pb * maxB * d);
   take_big(s ? s->Nxt : dummy, (long)pb * maxB * d);
@@ -231,6 +256,7 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
     s->Rf = nullptr;
   }
   if (big_doubles) *big_doubles = boff;
+  if (lng_doubles) *lng_doubles = loff;
   if (s) {
     s->sbC = pb * maxB;
     s->sbX = pa * maxB;
@@ -239,9 +265,9 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   return off;
 }
 
-// Work buffers of the QR-free FP64 sweep under layout fl: small ones and the placed matrix buffers from
-// base on, the others from big on (sizes as above; no Householder buffers, no proposal).  Returns
-// the doubles of shared memory; *big_doubles (if given) the others.
+// Work buffers of the QR-free FP64 sweep under layout fl: small ones and the placed buffers from base
+// on, the others from big on (sizes as above; no Householder buffers, no proposal); tables that are
+// not placed: nullptr.  Returns the doubles of shared memory; *big_doubles (if given) the others.
 __host__ __device__ inline long free_doubles(int L, int nC, int maxB, int G, int nJ, int pa, int pb,
                                              const FreeLayout &fl, Smem *s, double *base, double *big, long *big_doubles = nullptr) {
   long off = 0, boff = 0;
@@ -258,45 +284,42 @@ __host__ __device__ inline long free_doubles(int L, int nC, int maxB, int G, int
   x.Cm = take(16);
   x.O1 = take(4);
   x.O2 = take(4);
-  x.pdf = take((G + 31) & ~31);
   x.sc = take(16);
-  x.tabU = take(16L * nJ);
-  x.tabVT = take(16L * nJ);
-  x.tabSq = take(4L * nJ);
-  auto ints = [&](int n) { return reinterpret_cast<int *>(take((n + 1) / 2)); };
-  auto longs = [&](int n) { return reinterpret_cast<long *>(take(n)); };
-  x.aT = ints(L + 1);
-  x.bS = ints(L + 1);
-  x.site_c0 = ints(L + 1);
-  x.cp_j = ints(nC);
-  x.cp_q = ints(nC);
-  x.eopen = ints(L);
-  x.ech_off = ints(L + 1);
-  x.toff = longs(L);
-  x.roff = longs(L + 1);
-  x.zoff = longs(L);
-  {
-    double *a = take(L), *b = take((L + 1) / 2), *c = take((L + 1) / 2);
-    set_lists(x, a, b, c, take(1));
-  }
-  x.bW = ints(L + 1);
-  x.woff = longs(L);
   x.wsel = reinterpret_cast<int *>(take(1));
-  x.sbC = pb * maxB;
-  x.sbX = pa * maxB;
-  x.nx = fl.nx;
   auto place = [&](int k, long n) {
     if (fl.place >> k & 1u) return take(n);
     double *q = big + boff;
     boff += (n + 3) & ~3L;
     return q;
   };
+  auto table = [&](int k, long n) { return fl.place >> k & 1u ? take(n) : nullptr; };
+  auto ints = [&](int k, int n) { return reinterpret_cast<int *>(table(k, (n + 1) / 2)); };
+  auto longs = [&](int k, int n) { return reinterpret_cast<long *>(table(k, n)); };
+  x.tabU = table(kBufTab, 16L * nJ);
+  x.tabVT = table(kBufTab, 16L * nJ);
+  x.tabSq = table(kBufTab, 4L * nJ);
+  x.aT = ints(kBufSites, L + 1);
+  x.bS = ints(kBufSites, L + 1);
+  x.site_c0 = ints(kBufSites, L + 1);
+  x.eopen = ints(kBufSites, L);
+  x.ech_off = ints(kBufSites, L + 1);
+  x.toff = longs(kBufSites, L);
+  x.roff = longs(kBufSites, L + 1);
+  x.zoff = longs(kBufSites, L);
+  x.cp_j = ints(kBufCoup, nC);
+  x.cp_q = ints(kBufCoup, nC);
+  set_pdf(x, L, place(kBufPdf, pdf_doubles(L, G, true)), true);
+  x.bW = reinterpret_cast<int *>(place(kBufDims, (L + 2) / 2));
+  x.woff = reinterpret_cast<long *>(place(kBufDims, L));
+  x.sbC = pb * maxB;
+  x.sbX = pa * maxB;
+  x.nx = fl.nx;
   x.Xb = place(kBufXb, (long)x.sbX * fl.nx);
   x.Nxt = place(kBufNxt, (long)x.sbC * d);
   x.Cen = place(kBufCen, (long)x.sbC * d);
   x.Lenv = place(kBufLenv, x.sbX);
   x.Nl = place(kBufNl, (long)pb * maxB);
-  x.grid = place(kBufGrid, 4L * G);
+  x.grid = table(kBufGrid, 4L * G);
   x.Pb = place(kBufPb, (long)x.sbX * kN2);
   if (s) *s = x;
   if (big_doubles) *big_doubles = boff;
@@ -304,18 +327,25 @@ __host__ __device__ inline long free_doubles(int L, int nC, int maxB, int G, int
 }
 
 // The same buffers for the mixed-precision sweep: FP64 small buffers as above, FP32 matrix
-// buffers, no QR panel (that sweep is QR-free).  Sizes in bytes; *big_floats (if given)
-// receives the size of the matrix buffers in floats.
+// buffers, no QR panel (that sweep is QR-free).  Sizes in bytes; *big_floats and *lng_doubles (if
+// given) receive the sizes of the matrix buffers in floats and of the long ones in doubles.
 __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G, int pa, int pb,
                                                SmemT<float> *s, double *base, float *big = nullptr,
-                                               long *big_floats = nullptr, bool mlp = false) {
+                                               long *big_floats = nullptr, bool mlp = false, double *lng = nullptr,
+                                               long *lng_doubles = nullptr) {
   (void)maxA;  // the blocks are sized by the padded pa, pb
-  long off = 0, boff = 0;  // doubles of the small buffers; floats of the matrix buffers
+  long off = 0, boff = 0, loff = 0;  // doubles of the small buffers; floats of the matrix buffers; doubles of the long ones
   double *dummy;
   float *fdummy;
   auto take = [&](double *&p, long n) {
     if (s) p = base + off;
     off += (n + 3) & ~3L;
+  };
+  auto take_long = [&](long n) {
+    const long r = (n + 3) & ~3L;
+    double *p = lng ? lng + loff : base + off;
+    (lng ? loff : off) += r;
+    return p;
   };
   const int d = kMaxD;
   off += kTableDoubles + kArgDoubles;
@@ -326,15 +356,13 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
   take(s ? s->Cm : dummy, 16);
   take(s ? s->O1 : dummy, 4);
   take(s ? s->O2 : dummy, 4);
-  take(s ? s->pdf : dummy, (G + 31) & ~31);
   take(s ? s->sc : dummy, 16);
   {
-    double *b, *o, *q, *m;
-    take(b, (L + 2) / 2);
-    take(o, L);
-    take(q, 1);
-    take(m, mlp ? 400 : 0);
+    double *x = take_long(pdf_doubles(L, G, true)), *b = take_long((L + 2) / 2), *o = take_long(L), *q = nullptr, *m = nullptr;
+    take(s ? q : dummy, 1);
+    take(s ? m : dummy, mlp ? 400 : 0);
     if (s) {
+      set_pdf(*s, L, x, true);
       s->bW = reinterpret_cast<int *>(b);
       s->woff = reinterpret_cast<long *>(o);
       s->wsel = reinterpret_cast<int *>(q);
@@ -342,14 +370,6 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
     }
   }
   take(s ? s->qprop : dummy, mlp ? G : 0);
-  {
-    double *a, *b, *c, *e;
-    take(a, L);
-    take(b, (L + 1) / 2);
-    take(c, (L + 1) / 2);
-    take(e, 1);
-    if (s) set_lists(*s, a, b, c, e);
-  }
   float *fbase = reinterpret_cast<float *>(base + off);
   long soff = 0;  // floats placed in shared memory after the small buffers
   auto take_big = [&](float *&p, long n) {
@@ -376,6 +396,7 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
     s->nx = d;
   }
   if (big_floats) *big_floats = boff;
+  if (lng_doubles) *lng_doubles = loff;
   return (long)sizeof(double) * off + (long)sizeof(float) * soff;
 }
 
@@ -400,17 +421,17 @@ __device__ __forceinline__ void global_tables(const Dev &p, SmemT<T> &s) {
 // Carve the work buffers of the calling CTA (shared memory, plus its global scratch when the
 // matrix buffers do not fit on chip).
 __device__ __forceinline__ void carve(const Dev &p, Smem &s, double *smem_raw) {
-  double *big = (p.gwoff >= 0) ? p.scratch + (long)blockIdx.x * p.scr_stride + p.gwoff : nullptr;
-  smem_doubles(p.L, p.maxA, p.maxB, p.G, p.pa, p.pb, p.pq, &s, smem_raw, big, nullptr,
-               p.prop_mode != 0 || p.prop_collect != 0);
+  double *scr = p.scratch + (long)blockIdx.x * p.scr_stride;
+  smem_doubles(p.L, p.maxA, p.maxB, p.G, p.pa, p.pb, p.pq, &s, smem_raw, p.gwoff >= 0 ? scr + p.gwoff : nullptr,
+               nullptr, p.prop_mode != 0 || p.prop_collect != 0, true, p.lwoff >= 0 ? scr + p.lwoff : nullptr);
   global_tables(p, s);
 }
 // Mixed precision: the CTA's scratch is read as floats with the same element offsets.
 __device__ __forceinline__ void carve(const Dev &p, SmemT<float> &s, double *smem_raw) {
-  float *big = (p.gwoff >= 0) ? reinterpret_cast<float *>(p.scratch) + (long)blockIdx.x * p.scr_stride + p.gwoff
-                              : nullptr;
-  smem_bytes_f32(p.L, p.maxA, p.maxB, p.G, p.pa, p.pb, &s, smem_raw, big, nullptr,
-                 p.prop_mode != 0 || p.prop_collect != 0);
+  float *scr = reinterpret_cast<float *>(p.scratch) + (long)blockIdx.x * p.scr_stride;
+  smem_bytes_f32(p.L, p.maxA, p.maxB, p.G, p.pa, p.pb, &s, smem_raw, p.gwoff >= 0 ? scr + p.gwoff : nullptr, nullptr,
+                 p.prop_mode != 0 || p.prop_collect != 0,
+                 p.lwoff_mixed >= 0 ? reinterpret_cast<double *>(scr + p.lwoff_mixed) : nullptr);
   global_tables(p, s);
 }
 
@@ -425,7 +446,29 @@ __device__ __forceinline__ void carve_shared(const Dev &p, double *smem_raw) {
     if constexpr (std::is_same<T, double>::value) {
       free_doubles(p.L, p.nC, p.maxB, p.G, p.nJ, p.pa, p.pb, p.fl, &s, smem_raw,
                    p.scratch + (long)blockIdx.x * p.scr_stride + p.fwoff);
-      if (!(p.fl.place >> kBufGrid & 1u)) s.grid = p.grid;
+      SmemT<T> host;
+      global_tables(p, host);
+      const unsigned at = p.fl.place;
+      if (!(at >> kBufGrid & 1u)) s.grid = host.grid;
+      if (!(at >> kBufTab & 1u)) {
+        s.tabU = host.tabU;
+        s.tabSq = host.tabSq;
+        s.tabVT = host.tabVT;
+      }
+      if (!(at >> kBufCoup & 1u)) {
+        s.cp_j = host.cp_j;
+        s.cp_q = host.cp_q;
+      }
+      if (!(at >> kBufSites & 1u)) {
+        s.aT = host.aT;
+        s.bS = host.bS;
+        s.site_c0 = host.site_c0;
+        s.eopen = host.eopen;
+        s.ech_off = host.ech_off;
+        s.toff = host.toff;
+        s.roff = host.roff;
+        s.zoff = host.zoff;
+      }
     } else {
       carve(p, s, smem_raw);
     }
@@ -439,20 +482,27 @@ __device__ __forceinline__ void carve_shared(const Dev &p, double *smem_raw) {
       for (int q = threadIdx.x; q < n; q += blockDim.x) const_cast<V *>(dst)[q] = from[q];
     };
     const int L = p.L;
-    if (s.grid != p.grid) copy(s.grid, p.grid, 4 * p.G);
-    copy(s.tabU, p.tabU, 16 * p.nJ);
-    copy(s.tabVT, p.tabVT, 16 * p.nJ);
-    copy(s.tabSq, p.tabSq, 4 * p.nJ);
-    copy(s.aT, p.aT, L + 1);
-    copy(s.bS, p.bW, L + 1);
-    copy(s.site_c0, p.site_c0, L + 1);
-    copy(s.cp_j, p.cp_j, p.nC);
-    copy(s.cp_q, p.cp_q, p.nC);
-    copy(s.eopen, p.eopen, L);
-    copy(s.ech_off, p.ech_off, L + 1);
-    copy(s.toff, p.toff, L);
-    copy(s.roff, p.roff, L + 1);
-    copy(s.zoff, p.zoff, L);
+    const unsigned at = p.fl.place;
+    if (at >> kBufGrid & 1u) copy(s.grid, p.grid, 4 * p.G);
+    if (at >> kBufTab & 1u) {
+      copy(s.tabU, p.tabU, 16 * p.nJ);
+      copy(s.tabVT, p.tabVT, 16 * p.nJ);
+      copy(s.tabSq, p.tabSq, 4 * p.nJ);
+    }
+    if (at >> kBufCoup & 1u) {
+      copy(s.cp_j, p.cp_j, p.nC);
+      copy(s.cp_q, p.cp_q, p.nC);
+    }
+    if (at >> kBufSites & 1u) {
+      copy(s.aT, p.aT, L + 1);
+      copy(s.bS, p.bW, L + 1);
+      copy(s.site_c0, p.site_c0, L + 1);
+      copy(s.eopen, p.eopen, L);
+      copy(s.ech_off, p.ech_off, L + 1);
+      copy(s.toff, p.toff, L);
+      copy(s.roff, p.roff, L + 1);
+      copy(s.zoff, p.zoff, L);
+    }
     __syncthreads();
   }
 }
