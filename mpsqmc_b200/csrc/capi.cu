@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <random>
+#include <set>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -456,9 +457,6 @@ int layout_free(mpsqmc_ctx *c, bool force_global) {
   c->smem_bytes_free = bytes(f, &big);
   c->fwoff = (c->scr_base + 31) & ~31L;
   c->scr_stride = std::max(c->scr_stride, (c->fwoff + big + 31) & ~31L);
-  for (const void *k : {(const void *)mq::walker_step_kernel_fp64<true>, (const void *)mq::walker_step_kernel_fp64<false>,
-                        (const void *)mq::energy_general_kernel})
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_bytes_free));
   c->free_threads = threads;
   int occ = 1;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mq::walker_step_kernel_fp64<false>, threads, c->smem_bytes_free));
@@ -466,6 +464,30 @@ int layout_free(mpsqmc_ctx *c, bool force_global) {
   int n = std::max(1, std::min(occ, ctas));
   while (n > 1 && (size_t)n * c->sm_count * c->scr_stride * sizeof(double) > c->total_mem / 16) --n;
   c->max_ctas_free = n * c->sm_count;
+  return 0;
+}
+
+// Every kernel's dynamic shared memory may reach the device's limit: the attribute belongs to the
+// process, so it must not be one context's size (a launch is given its own).  Set at the first create
+// on a device.
+int allow_shared_memory(int device, size_t optin) {
+  static std::mutex m;
+  static std::set<int> done;
+  std::lock_guard<std::mutex> lk(m);
+  if (done.count(device)) return 0;
+  const void *kernels[] = {
+      (const void *)mq::walker_step_kernel, (const void *)mq::set_overlap_kernel, (const void *)mq::energy_kernel,
+      (const void *)mq::walker_step_general_kernel<true>, (const void *)mq::walker_step_general_kernel<false>,
+      (const void *)mq::legacy_step_kernel, (const void *)mq::walker_step_kernel_fp64<true>,
+      (const void *)mq::walker_step_kernel_fp64<false>, (const void *)mq::energy_general_kernel,
+      (const void *)mq::walker_step_mixed_kernel<1, true>, (const void *)mq::walker_step_mixed_kernel<3, true>,
+      (const void *)mq::walker_step_mixed_kernel<1, false>, (const void *)mq::walker_step_mixed_kernel<3, false>};
+  for (const void *k : kernels) {
+    cudaFuncAttributes a;
+    CK(cudaFuncGetAttributes(&a, k));
+    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(optin - a.sharedSizeBytes)));
+  }
+  done.insert(device);
   return 0;
 }
 
@@ -488,11 +510,6 @@ int layout_workspace(mpsqmc_ctx *c, bool force_global) {
   c->lwoff = lng ? base + ((nbig + 31) & ~31L) : -1;
   c->scr_stride = lng ? c->lwoff + ((nlong + 31) & ~31L) : global ? base + ((nbig + 31) & ~31L) : base;
   c->global_work = global;
-  const void *kernels[] = {(const void *)mq::walker_step_kernel, (const void *)mq::set_overlap_kernel,
-                           (const void *)mq::energy_kernel, (const void *)mq::walker_step_general_kernel<true>,
-                           (const void *)mq::walker_step_general_kernel<false>, (const void *)mq::legacy_step_kernel};
-  for (const void *k : kernels)
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_bytes));
   int occ = 1;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mq::walker_step_kernel, mq::kThreads, c->smem_bytes));
   c->max_ctas = std::max(1, occ) * c->sm_count;
@@ -511,10 +528,6 @@ int layout_workspace(mpsqmc_ctx *c, bool force_global) {
   c->smem_bytes_mixed = mixed_bytes(lng_f, &big_floats, &nlong);
   c->lwoff_mixed = lng_f ? base + ((big_floats + 31) & ~31L) : -1;
   if (lng_f) c->scr_stride = std::max(c->scr_stride, c->lwoff_mixed + ((2 * nlong + 31) & ~31L));
-  const void *mk[] = {(const void *)mq::walker_step_mixed_kernel<1, true>, (const void *)mq::walker_step_mixed_kernel<3, true>,
-                      (const void *)mq::walker_step_mixed_kernel<1, false>, (const void *)mq::walker_step_mixed_kernel<3, false>};
-  for (const void *k : mk)
-    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->smem_bytes_mixed));
   int occm = 1;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occm, mq::walker_step_mixed_kernel<3, true>, mq::kThreads,
                                                    c->smem_bytes_mixed));
@@ -753,7 +766,8 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
   if (c->maxB > mq::kThreads / 2)
     return bail(fail(MPSQMC_E_UNSUPPORTED, "walker bond dimension above 128 (one QR column group per warp)"));
   {
-    const int rc = layout_workspace(c, false);
+    int rc = allow_shared_memory(c->device, prop.sharedMemPerBlockOptin);
+    if (!rc) rc = layout_workspace(c, false);
     if (rc) return bail(rc);
   }
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
