@@ -157,10 +157,8 @@ __global__ void __launch_bounds__(kThreads, 1) compress_kernel(Dev p, const int 
         const int m = DL * d, n = DR * d;
         double *Al = Wk + p.woff[k], *Ar = Wk + p.woff[k + 1];
         // Theta (TwoSiteObject.cpp:111-115, 126-134)
-        for (int il = 0; il < d; ++il)
-          for (int ir = 0; ir < d; ++ir)
-            cta_gemm(DL, DR, DM, 1.0, Al + (long)il * DL * DM, DL, false, Ar + (long)ir * DM * DR, DM, false, 0.0,
-                     T + DL * il + (long)m * DR * ir, m);
+        gemm_g<0>(DL, DR, DM, cols(Al, DL, (long)DL * DM), d, rows(Ar, DM, (long)DM * DR), d, 1, false, T, m, DL,
+                  (long)m * DR);
         __syncthreads();
         const bool tall = m >= n;
         double *Mx = T;

@@ -375,26 +375,6 @@ static __device__ __noinline__ void cta_gemm_small() {
   }
 }
 
-// C (M x N, ldc) = op(A) * op(B) + (beta ? C : 0), op(A) M x K, op(B) K x N; any M, N, K >= 0.
-//   ta == false: A[m + lda*k];  ta == true: A[k + lda*m]
-//   tb == false: B[k + ldb*n];  tb == true: B[n + ldb*k]  (not both)
-// Two calls with the same M, N may accumulate into C without a barrier.
-static __device__ __forceinline__ void cta_gemm(int M, int N, int K, double alpha, const double *A, int lda, bool ta,
-                                                const double *B, int ldb, bool tb, double beta, double *C, int ldc) {
-  (void)alpha;  // 1 everywhere
-  const bool add = beta != 0.0;
-  if (ta) {
-    set_op(M, N, K, rows(A, lda), 1, rows(B, ldb), 1, 1, add, C, ldc, 0, 0);
-    cta_gemm_groups<true, true>();
-  } else if (tb) {
-    set_op(M, N, K, cols(A, lda), 1, cols(B, ldb), 1, 1, add, C, ldc, 0, 0);
-    cta_gemm_groups<false, false>();
-  } else {
-    set_op(M, N, K, cols(A, lda), 1, rows(B, ldb), 1, 1, add, C, ldc, 0, 0);
-    cta_gemm_groups<false, true>();
-  }
-}
-
 // ---------------------------------------------------------------------------------------------
 // FP32 storage, TF32 tensor cores (the mixed-precision sweep)
 //

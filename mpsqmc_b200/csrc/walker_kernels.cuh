@@ -610,15 +610,11 @@ static __device__ void env_update(const Dev &p, Smem &s, const double *B, int al
                            double Jprev, bool first) {
   const int d = kMaxD, lda = p.maxA, fstride = p.maxA * p.maxB;
   // X[tau] = Lenv * T[tau]      (al x br)
-  for (int tau = 0; tau < d; ++tau)
-    cta_gemm(al, br, bl, 1.0, s.Lenv, p.pa, false, T + tau * ss, cs, false, 0.0, s.Xb + tau * s.sbX,
-             p.pa);
+  gemm_g<0>(al, br, bl, cols(s.Lenv, p.pa), 1, rows(T, cs, ss), d, 1, false, s.Xb, p.pa, 0, s.sbX);
   __syncthreads();
   // P[sigma + d*tau] = B[sigma]^T X[tau]   (ar x br)
-  for (int sg = 0; sg < d; ++sg)
-    for (int tau = 0; tau < d; ++tau)
-      cta_gemm(ar, br, al, 1.0, B + (long)sg * al * ar, al, true, s.Xb + tau * s.sbX, p.pa, false,
-               0.0, s.Pb + (sg + d * tau) * s.sbX, p.pa);
+  gemm_g<0>(ar, br, al, rows(B, al, (long)al * ar), d, rows(s.Xb, p.pa, s.sbX), d, 1, false, s.Pb, p.pa, s.sbX,
+            d * s.sbX);
   __syncthreads();
   // Lenv' and the operator channels opened on this site; field closes immediately.
   for (int q = threadIdx.x; q < ar * br; q += kThreads) {
@@ -643,30 +639,27 @@ static __device__ void env_update(const Dev &p, Smem &s, const double *B, int al
   __syncthreads();
   if (first) return;
   // Fdone' += sum_s B[s]^T ( sum_t G_st T[t] ),
-  // G_st = delta_st Fdone + Jprev (Sx(s,t) F_Sx - iSy(s,t) F_iSy + Sz(s,t) F_Sz)
-  for (int sg = 0; sg < d; ++sg) {
-    for (int q = threadIdx.x; q < al * bl; q += kThreads) {
-      const int r = q % al, c = q / al;
-      const double fd = Fcur[0 * fstride + r + lda * c];
-      const double fx = Fcur[1 * fstride + r + lda * c];
-      const double fy = Fcur[2 * fstride + r + lda * c];
-      const double fz = Fcur[3 * fstride + r + lda * c];
-      for (int tau = 0; tau < d; ++tau) {
-        const int k = sg + d * tau;
-        const double g = ((sg == tau) ? fd : 0.0) +
-                         Jprev * (p.opSx[k] * fx - p.opISy[k] * fy + p.opSz[k] * fz);
-        s.Xb[tau * s.sbX + r + p.pa * c] = g;
-      }
+  // G_st = delta_st Fdone + Jprev (Sx(s,t) F_Sx - iSy(s,t) F_iSy + Sz(s,t) F_Sz): G_0t in Xb[t], G_1t in
+  // Pb[t] (the branches are no longer needed), sum_t G_st T[t] in Pb[2 + s]
+  for (int q = threadIdx.x; q < al * bl; q += kThreads) {
+    const int r = q % al, c = q / al;
+    const double fd = Fcur[0 * fstride + r + lda * c];
+    const double fx = Fcur[1 * fstride + r + lda * c];
+    const double fy = Fcur[2 * fstride + r + lda * c];
+    const double fz = Fcur[3 * fstride + r + lda * c];
+#pragma unroll
+    for (int k = 0; k < kN2; ++k) {
+      const int sg = k % d, tau = k / d;
+      (sg == 0 ? s.Xb : s.Pb)[tau * s.sbX + r + p.pa * c] =
+          ((sg == tau) ? fd : 0.0) + Jprev * (p.opSx[k] * fx - p.opISy[k] * fy + p.opSz[k] * fz);
     }
-    __syncthreads();
-    cta_gemm(al, br, bl, 1.0, s.Xb, p.pa, false, T, cs, false, 0.0, s.Qt, p.pa);
-    for (int tau = 1; tau < d; ++tau)
-      cta_gemm(al, br, bl, 1.0, s.Xb + tau * s.sbX, p.pa, false, T + tau * ss, cs, false, 1.0, s.Qt,
-               p.pa);
-    __syncthreads();
-    cta_gemm(ar, br, al, 1.0, B + (long)sg * al * ar, al, true, s.Qt, p.pa, false, 1.0, Fnxt, lda);
-    __syncthreads();
   }
+  __syncthreads();
+  gemm_g<0>(al, br, bl, cols(s.Xb, p.pa, s.Pb - s.Xb, s.sbX), d, rows(T, cs, 0, ss), 1, d, false, s.Pb + d * s.sbX, p.pa,
+            s.sbX);
+  __syncthreads();
+  gemm_g<0>(ar, br, al, rows(B, al, 0, (long)al * ar), 1, rows(s.Pb + d * s.sbX, p.pa, 0, s.sbX), 1, d, true, Fnxt, lda);
+  __syncthreads();
 }
 
 // Translation units that only need the device helpers above define MQ_DEVICE_ONLY, so that
@@ -708,20 +701,12 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev p) {
         const double *Rn = scr + p.roff[k + 1], *Nn = scr + p.nroff[k + 1];
         double *Rk = scr + p.roff[k], *Nk = scr + p.nroff[k];
         const double *Bk = p.trial + p.toff[k];
-        for (int sg = 0; sg < d; ++sg) {
-          // Y[s] = R[k+1] A_k[s]^T (ar x bl),  Z[s] = N[k+1] A_k[s]^T (br x bl)
-          cta_gemm(ar, bl, br, 1.0, Rn, ar, false, s.Nxt + sg * s.sbC, p.pb, true, 0.0,
-                   s.Xb + sg * s.sbX, p.pa);
-          cta_gemm(br, bl, br, 1.0, Nn, br, false, s.Nxt + sg * s.sbC, p.pb, true, 0.0,
-                   s.Pb + sg * s.sbX, p.pa);
-        }
+        // Y[s] = R[k+1] A_k[s]^T (ar x bl),  Z[s] = N[k+1] A_k[s]^T (br x bl)
+        gemm_g<0>(ar, bl, br, cols(Rn, ar), 1, cols(s.Nxt, p.pb, s.sbC), d, 1, false, s.Xb, p.pa, 0, s.sbX);
+        gemm_g<0>(br, bl, br, cols(Nn, br), 1, cols(s.Nxt, p.pb, s.sbC), d, 1, false, s.Pb, p.pa, 0, s.sbX);
         __syncthreads();
-        for (int sg = 0; sg < d; ++sg) {
-          cta_gemm(al, bl, ar, 1.0, Bk + (long)sg * al * ar, al, false, s.Xb + sg * s.sbX, p.pa, false,
-                   sg == 0 ? 0.0 : 1.0, Rk, al);
-          cta_gemm(bl, bl, br, 1.0, s.Nxt + sg * s.sbC, p.pb, false, s.Pb + sg * s.sbX, p.pa, false,
-                   sg == 0 ? 0.0 : 1.0, Nk, bl);
-        }
+        gemm_g<0>(al, bl, ar, cols(Bk, al, 0, (long)al * ar), 1, rows(s.Xb, p.pa, 0, s.sbX), 1, d, false, Rk, al);
+        gemm_g<0>(bl, bl, br, cols(s.Nxt, p.pb, 0, s.sbC), 1, rows(s.Pb, p.pa, 0, s.sbX), 1, d, false, Nk, bl);
         __syncthreads();
       }
       // centre = site 0 (1 x b1): ||phi||^2 = sum_s C[s] N[1] C[s]^T, ov = sum_s B_0[s] R[1] C[s]^T
@@ -769,38 +754,16 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev p) {
         const int jq = p.bond_j[i];
         const double *U = p.tabU + 16 * jq, *Sq = p.tabSq + 4 * jq, *VT = p.tabVT + 16 * jq;
         // left branches P[s + d t] = B_i[s]^T Lenv C[t]
-        for (int tau = 0; tau < d; ++tau)
-          cta_gemm(al, br, bl, 1.0, s.Lenv, p.pa, false, s.Cen + tau * s.sbC, p.pb, false, 0.0,
-                   s.Xb + tau * s.sbX, p.pa);
+        gemm_g<0>(al, br, bl, cols(s.Lenv, p.pa), 1, rows(s.Cen, p.pb, s.sbC), d, 1, false, s.Xb, p.pa, 0, s.sbX);
         __syncthreads();
-        for (int sg = 0; sg < d; ++sg)
-          for (int tau = 0; tau < d; ++tau)
-            cta_gemm(ar, br, al, 1.0, Bi + (long)sg * al * ar, al, true, s.Xb + tau * s.sbX, p.pa,
-                     false, 0.0, s.Pb + (sg + d * tau) * s.sbX, p.pa);
+        gemm_g<0>(ar, br, al, rows(Bi, al, (long)al * ar), d, rows(s.Xb, p.pa, s.sbX), d, 1, false, s.Pb, p.pa, s.sbX,
+                  d * s.sbX);
         __syncthreads();
-        // right branches Y[t'] = R[i+2] N[t']^T, Q = B_j[s'] Y[t'], closures M[p + 4q]
+        // right branches Y[t'] = R[i+2] N[t']^T, closures M[p + 4q] with B_j[s'] Y[t']
         const double *R2 = scr + p.roff[i + 2];
-        for (int tau = 0; tau < d; ++tau)
-          cta_gemm(a2, br, b2, 1.0, R2, a2, false, s.Nxt + tau * s.sbC, p.pb, true, 0.0,
-                   s.Xb + tau * s.sbX, p.pa);
+        gemm_g<0>(a2, br, b2, cols(R2, a2), 1, cols(s.Nxt, p.pb, s.sbC), d, 1, false, s.Xb, p.pa, 0, s.sbX);
         __syncthreads();
-        for (int sg = 0; sg < d; ++sg)
-          for (int tau = 0; tau < d; ++tau) {
-            cta_gemm(ar, br, a2, 1.0, Bj + (long)sg * ar * a2, ar, false, s.Xb + tau * s.sbX, p.pa,
-                     false, 0.0, s.Qt, p.pa);
-            __syncthreads();
-            double v[4] = {0.0, 0.0, 0.0, 0.0};
-            for (int q = tid; q < ar * br; q += kThreads) {
-              const int r = q % ar, cc = q / ar;
-              const double qv = s.Qt[r + p.pa * cc];
-#pragma unroll
-              for (int k = 0; k < 4; ++k) v[k] += s.Pb[k * s.sbX + r + p.pa * cc] * qv;
-            }
-            cta_sum4(v, s.red);
-            if (tid == 0)
-              for (int k = 0; k < 4; ++k) s.M[k + 4 * (sg + d * tau)] = v[k];
-          }
-        __syncthreads();
+        cta_closure16<0>(ar, br, a2, Bj, ar, ar * a2, s.Xb, p.pa, s.sbX, s.Pb, p.pa, s.sbX, s.red, s.M);
         // C[k + 4 l] = sqrt(s_k s_l) sum_{p,q} U[p + 4k] VT[l + 4q] M[p + 4q]
         if (tid < 16) {
           const int k = tid & 3, l = tid >> 2;
@@ -884,9 +847,7 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev p) {
       __syncthreads();
       // move the centre: QR of site i, R into site i+1
       cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau, s.wv, s.red);
-      for (int sg = 0; sg < d; ++sg)
-        cta_gemm(br, b2, br, 1.0, s.Rf, p.pb, false, s.Nxt + sg * s.sbC, p.pb, false, 0.0,
-                 s.Cen + sg * s.sbC, p.pb);
+      gemm_g<0>(br, b2, br, cols(s.Rf, p.pb), 1, rows(s.Nxt, p.pb, s.sbC), d, 1, false, s.Cen, p.pb, 0, s.sbC);
       // site i <- Q
       {
         double *Wi = W + s.woff[i];
@@ -899,9 +860,7 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev p) {
       if (c >= 0) {
         // ||B(x) phi||^2 = sum_s tr(C[s] N[i+2] C[s]^T): sites < i+1 are orthonormal now
         const double *N2 = scr + p.nroff[i + 2];
-        for (int sg = 0; sg < d; ++sg)
-          cta_gemm(br, b2, b2, 1.0, s.Cen + sg * s.sbC, p.pb, false, N2, b2, false, 0.0, s.Xb + sg * s.sbX,
-                   p.pa);
+        gemm_g<0>(br, b2, b2, cols(s.Cen, p.pb, s.sbC), d, rows(N2, b2), 1, 1, false, s.Xb, p.pa, s.sbX);
         __syncthreads();
         double part = 0.0;
         for (int q = tid; q < br * b2 * d; q += kThreads) {
@@ -987,9 +946,7 @@ __global__ void __launch_bounds__(kThreads, 1) set_overlap_kernel(Dev p) {
         const int b2 = s.bW[k + 2];
         load_site(s.Nxt, p.pb, s.sbC, W + s.woff[k + 1], br, b2);
         __syncthreads();
-        for (int sg = 0; sg < d; ++sg)
-          cta_gemm(br, b2, br, 1.0, s.Rf, p.pb, false, s.Nxt + sg * s.sbC, p.pb, false, 0.0,
-                   s.Cen + sg * s.sbC, p.pb);
+        gemm_g<0>(br, b2, br, cols(s.Rf, p.pb), 1, rows(s.Nxt, p.pb, s.sbC), d, 1, false, s.Cen, p.pb, 0, s.sbC);
       }
       __syncthreads();
     }
@@ -1000,16 +957,9 @@ __global__ void __launch_bounds__(kThreads, 1) set_overlap_kernel(Dev p) {
       const int al = p.aT[k], ar = p.aT[k + 1], bl = s.bW[k], br = s.bW[k + 1];
       const double *A = W + s.woff[k];
       const double *B = p.trial + p.toff[k];
-      for (int sg = 0; sg < d; ++sg)
-        cta_gemm(al, br, bl, 1.0, s.Lenv, p.pa, false, A + (long)sg * bl * br, bl, false, 0.0,
-                 s.Xb + sg * s.sbX, p.pa);
+      gemm_g<0>(al, br, bl, cols(s.Lenv, p.pa), 1, rows(A, bl, (long)bl * br), d, 1, false, s.Xb, p.pa, 0, s.sbX);
       __syncthreads();
-      cta_gemm(ar, br, al, 1.0, B, al, true, s.Xb, p.pa, false, 0.0, s.Qt, p.pa);
-      for (int sg = 1; sg < d; ++sg)
-        cta_gemm(ar, br, al, 1.0, B + (long)sg * al * ar, al, true, s.Xb + sg * s.sbX, p.pa, false,
-                 1.0, s.Qt, p.pa);
-      __syncthreads();
-      for (int q = tid; q < ar * br; q += kThreads) s.Lenv[(q % ar) + p.pa * (q / ar)] = s.Qt[(q % ar) + p.pa * (q / ar)];
+      gemm_g<0>(ar, br, al, rows(B, al, 0, (long)al * ar), 1, rows(s.Xb, p.pa, 0, s.sbX), 1, d, false, s.Lenv, p.pa);
       __syncthreads();
     }
     double ov = s.Lenv[0];
