@@ -39,6 +39,7 @@
 // energies in FP64; walkers stay FP64 in HBM).  The mixed sweep is always QR-free.
 #pragma once
 
+#include <cfloat>
 #include <type_traits>
 
 #include "proposal.cuh"
@@ -434,8 +435,7 @@ __device__ __forceinline__ void take_point(const Dev &p, SmemT<T> &s, int jq, in
 // cycles of a coupling on average).  The sum in front of a lane and the last running sum of the lane
 // before it are rounded differently; a uniform between the two goes to the next point of nonzero
 // probability (behind the last sum: to the last such point), as the sampled point's sum C x x has to
-// be positive.  Comparisons are those of the
-// serial scan: a NaN (the sum of the PDF is zero) ends it at the first point.
+// be positive.
 template <typename T>
 static __device__ __noinline__ void sample_grid(const Dev &p, SmemT<T> &s, int c, int jq) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -473,12 +473,14 @@ static __device__ __noinline__ void sample_grid(const Dev &p, SmemT<T> &s, int c
     for (int i = 0; i < per; ++i) {
       const double v = s.pdf[32 * i + lane];
       at += v;
-      const double x = at * pinv;
-      if (hit == per && !(x <= u) && (v > 0.0 || isnan(x))) hit = i;
+      if (hit == per && at * pinv > u && __double2hiint(v) != 0) hit = i;
     }
     const unsigned who = __ballot_sync(full, hit < per);
-    int count;
-    if (who) {
+    int count = 0;
+    if (!(pinv > 0.0 && pinv <= DBL_MAX)) {  // a sum that is zero, infinite or no number: as the serial scan ends
+      auto pdf = [&](int g) { return s.pdf[32 * (g % per) + g / per] * pinv; };
+      for (double cum = pdf(0); cum <= u && count < p.G - 1; cum += pdf(count)) ++count;
+    } else if (who) {
       const int src = __ffs(who) - 1;
       count = min(p.G - 1, src * per + __shfl_sync(full, hit, src));
     } else {  // u beyond the last sum by rounding: the last point of nonzero probability
