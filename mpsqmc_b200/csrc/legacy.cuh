@@ -37,10 +37,11 @@ __device__ __forceinline__ const double *legacy_op(const Dev &p, int code) {
 
 #ifndef MQ_DEVICE_ONLY
 
-__global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev p, LegacyDev lp) {
+__global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev args, LegacyDev lp) {
   extern __shared__ double smem_raw[];
-  Smem s;
-  carve(p, s, smem_raw);
+  carve_shared<double>(args, smem_raw);
+  const Dev &p = shared_args(smem_raw);
+  Smem &s = *reinterpret_cast<Smem *>(smem_raw);
   const int L = p.L, d = kMaxD, tid = threadIdx.x;
   const int N = *p.n_cur;
   double *scr = p.scratch + (long)blockIdx.x * p.scr_stride;
@@ -50,9 +51,12 @@ __global__ void __launch_bounds__(kThreads, 1) legacy_step_kernel(Dev p, LegacyD
     const int slot = p.slot_of[w];
     load_walker_dims(p, s, slot);
     double *W = p.walkers + (long)slot * p.wstride;
-    s.W = W;
-    s.scr = scr;
-    if (tid == 0) scr[p.roff[L]] = 1.0;
+    if (tid == 0) {
+      s.W = W;
+      s.scr = scr;
+      scr[p.roff[L]] = 1.0;
+    }
+    __syncthreads();
     for (int k = L - 1; k >= 1; --k) right_env_step<double>(p, s, k);
     if (tid == 0) s.Lenv[0] = 1.0;
     __syncthreads();

@@ -761,12 +761,10 @@ static __device__ double norm_from_centre(const Dev &p, SmemT<T> &s, int i, cons
 // and its training are compiled in.
 template <typename T, int NP, bool ZB, int QM, bool TR, bool LEARN>
 __device__ __forceinline__ void general_step(const Dev &args, double *smem_raw) {
-  const Dev &p = QM == 1 ? shared_args(smem_raw) : args;
+  const Dev &p = shared_args(smem_raw);
   constexpr bool kMixed = !std::is_same<T, double>::value;
-  SmemT<T> own;
-  SmemT<T> &s = QM == 1 ? *reinterpret_cast<SmemT<T> *>(smem_raw) : own;
-  if constexpr (QM != 1) carve(p, s, smem_raw);
-  else carve_shared<T>(args, smem_raw);
+  SmemT<T> &s = *reinterpret_cast<SmemT<T> *>(smem_raw);
+  carve_shared<T, QM == 1 && !kMixed>(args, smem_raw);
   const bool QF = QM == 1 || args.nloff >= 0;
   const bool traced = TR && args.trace != nullptr;
   const int L = p.L, d = kMaxD, tid = threadIdx.x;
@@ -776,7 +774,7 @@ __device__ __forceinline__ void general_step(const Dev &args, double *smem_raw) 
     {
       const int slot = p.slot_of[w];
       load_walker_dims(p, s, slot);
-      if (QM != 1 || tid == 0) {  // (the table is the thread's own, or the CTA's)
+      if (tid == 0) {
         T *scr = reinterpret_cast<T *>(p.scratch) + (long)blockIdx.x * p.scr_stride;
         const long fm = (long)p.maxA * p.maxB;
         s.w = w;
@@ -910,7 +908,7 @@ __device__ __forceinline__ void general_step(const Dev &args, double *smem_raw) 
         env_update_general<T, NP>(p, s, i, s.Cen, p.pb, s.sbC);
         finish_walker(p, s, i);
       }
-      if (QM != 1 || tid == 0) {  // the "done" channel changes places
+      if (tid == 0) {  // the "done" channel changes places
         T *f = s.Fd;
         s.Fd = s.Fdn;
         s.Fdn = f;
@@ -948,7 +946,7 @@ __global__ void __launch_bounds__(kThreads, 2) walker_step_mixed_kernel(Dev p) {
 __global__ void __launch_bounds__(32 * kMaxWarps, 1) energy_general_kernel(Dev args) {
   extern __shared__ double smem_raw[];
   Smem &s = *reinterpret_cast<Smem *>(smem_raw);
-  carve_shared<double>(args, smem_raw);
+  carve_shared<double, true>(args, smem_raw);
   const Dev &p = shared_args(smem_raw);
   const int L = p.L, tid = threadIdx.x;
   for (;;) {

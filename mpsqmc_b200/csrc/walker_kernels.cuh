@@ -155,10 +155,10 @@ struct SmemT {
 // s.sc: what the threads of a CTA hand one another (1-7: sampling), and the walker's running numbers
 enum : int { kScOv = 8, kScWt = 9, kScNorm = 10 };
 using Smem = SmemT<double>;
-// The QR-free sweeps keep this table and the kernel's arguments in shared memory, in front of the
+// The engine's kernels keep this table and their arguments in shared memory, in front of the
 // buffers: as registers of every thread, hoisted out of the loops over sites, they cost the
 // products their fragments (spilled around each call: 28 MB of local-memory traffic per walker
-// and step of the L = 64 chain).
+// and step of the L = 64 chain in the QR-free sweep).
 constexpr int kTableDoubles = 64, kArgDoubles = (sizeof(Dev) + 31) / 32 * 4;
 static_assert(sizeof(Smem) <= 8 * kTableDoubles, "buffer table");
 
@@ -192,10 +192,11 @@ __host__ inline long limit_doubles(int L, int maxB, int G, bool mlp) {
 // the GEMMs read them through L1/L2.  The small ones that grow with the chain or the grid go there
 // too (lng != nullptr) where they leave no room for the others.  Returns the doubles placed in
 // shared memory; *big_doubles and *lng_doubles (if given) receive the sizes of the matrix buffers
-// and of the long ones.  mlp: the learned proposal's buffers.
+// and of the long ones.  mlp: the learned proposal's buffers; engine: the buffers of the engine's
+// kernels, with their table and arguments in front (else those of env_update alone).
 __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, int pa, int pb, int pq,
                                               Smem *s, double *base, double *big = nullptr,
-                                              long *big_doubles = nullptr, bool mlp = false, bool qr = true,
+                                              long *big_doubles = nullptr, bool mlp = false, bool engine = true,
                                               double *lng = nullptr, long *lng_doubles = nullptr) {
   (void)maxA;  // the blocks are sized by the padded pa, pb
   long off = 0, boff = 0, loff = 0;
@@ -221,6 +222,7 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
     return p;
   };
   const int d = kMaxD;
+  if (engine) off += kTableDoubles + kArgDoubles;
   take(s ? s->red : dummy, 16 * kWarps);
   take(s ? s->tau : dummy, maxB);
   take(s ? s->wv : dummy, maxB);
@@ -230,11 +232,11 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   take(s ? s->O2 : dummy, 4);
   take(s ? s->sc : dummy, 16);
   {
-    double *x = take_long(pdf_doubles(L, G, qr)), *b = take_long((L + 2) / 2), *o = take_long(L), *q = nullptr, *m = nullptr;
+    double *x = take_long(pdf_doubles(L, G, engine)), *b = take_long((L + 2) / 2), *o = take_long(L), *q = nullptr, *m = nullptr;
     take(s ? q : dummy, 1);
     take(s ? m : dummy, mlp ? 400 : 0);
     if (s) {
-      set_pdf(*s, L, x, qr);
+      set_pdf(*s, L, x, engine);
       s->bW = reinterpret_cast<int *>(b);
       s->woff = reinterpret_cast<long *>(o);
       s->wsel = reinterpret_cast<int *>(q);
@@ -248,7 +250,7 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   take_big(s ? s->Xb : dummy, (long)pa * maxB * d);
   take_big(s ? s->Pb : dummy, (long)pa * maxB * kN2);
   take_big(s ? s->Qt : dummy, (long)pa * maxB);
-  if (qr) {  // the Householder panel and R factor, last: the QR-free sweep goes without them
+  if (engine) {  // the Householder panel and R factor, last: the QR-free sweep goes without them
     take_big(s ? s->QRb : dummy, (long)pq * maxB);
     take_big(s ? s->Rf : dummy, (long)pb * maxB);
   } else if (s) {
@@ -435,15 +437,15 @@ __device__ __forceinline__ void carve(const Dev &p, SmemT<float> &s, double *sme
   global_tables(p, s);
 }
 
-// The QR-free sweeps: table and arguments into shared memory.  Ends with a barrier.
-template <typename T>
+// Table and arguments into shared memory.  FREE: the QR-free FP64 sweep's layout.  Ends with a barrier.
+template <typename T, bool FREE = false>
 __device__ __forceinline__ void carve_shared(const Dev &p, double *smem_raw) {
   const int *src = reinterpret_cast<const int *>(&p);
   int *dst = reinterpret_cast<int *>(smem_raw + kTableDoubles);
   for (int q = threadIdx.x; q < (int)(sizeof(Dev) / sizeof(int)); q += blockDim.x) dst[q] = src[q];
   if (threadIdx.x == 0) {
     SmemT<T> s;
-    if constexpr (std::is_same<T, double>::value) {
+    if constexpr (FREE) {
       free_doubles(p.L, p.nC, p.maxB, p.G, p.nJ, p.pa, p.pb, p.fl, &s, smem_raw,
                    p.scratch + (long)blockIdx.x * p.scr_stride + p.fwoff);
       SmemT<T> host;
@@ -475,7 +477,7 @@ __device__ __forceinline__ void carve_shared(const Dev &p, double *smem_raw) {
     *reinterpret_cast<SmemT<T> *>(smem_raw) = s;
   }
   __syncthreads();
-  if constexpr (std::is_same<T, double>::value) {
+  if constexpr (FREE) {
     const Smem &s = *reinterpret_cast<Smem *>(smem_raw);
     auto copy = [&](const auto *dst, const auto *from, int n) {
       using V = std::remove_const_t<std::remove_reference_t<decltype(*dst)>>;
@@ -669,10 +671,11 @@ static __device__ void env_update(const Dev &p, Smem &s, const double *B, int al
 // ---------------------------------------------------------------------------------------------
 // The walker-step kernel
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev p) {
+__global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev args) {
   extern __shared__ double smem_raw[];
-  Smem s;
-  carve(p, s, smem_raw);
+  carve_shared<double>(args, smem_raw);
+  const Dev &p = shared_args(smem_raw);
+  Smem &s = *reinterpret_cast<Smem *>(smem_raw);
   const int L = p.L, d = kMaxD, tid = threadIdx.x;
   const int N = *p.n_cur;
   double *scr = p.scratch + (long)blockIdx.x * p.scr_stride;
@@ -916,10 +919,11 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev p) {
 // Walker::setOverlap exactly as the reference does it (Walker.cpp:54-66): Householder
 // LeftNormalize (MPSstate.cpp:216-229), overlap <Psi_T|phi>, ChangePhase if negative.
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 1) set_overlap_kernel(Dev p) {
+__global__ void __launch_bounds__(kThreads, 1) set_overlap_kernel(Dev args) {
   extern __shared__ double smem_raw[];
-  Smem s;
-  carve(p, s, smem_raw);
+  carve_shared<double>(args, smem_raw);
+  const Dev &p = shared_args(smem_raw);
+  Smem &s = *reinterpret_cast<Smem *>(smem_raw);
   const int L = p.L, d = kMaxD, tid = threadIdx.x;
   const int N = *p.n_cur;
   for (int w = next_walker(s, p.ctr + kCtrSetOverlap); w < N; w = next_walker(s, p.ctr + kCtrSetOverlap)) {
@@ -975,10 +979,11 @@ __global__ void __launch_bounds__(kThreads, 1) set_overlap_kernel(Dev p) {
 }
 
 // <Psi_T|H|phi> / overlap for every walker, walker tensors taken as stored (any gauge).
-__global__ void __launch_bounds__(kThreads, 1) energy_kernel(Dev p) {
+__global__ void __launch_bounds__(kThreads, 1) energy_kernel(Dev args) {
   extern __shared__ double smem_raw[];
-  Smem s;
-  carve(p, s, smem_raw);
+  carve_shared<double>(args, smem_raw);
+  const Dev &p = shared_args(smem_raw);
+  Smem &s = *reinterpret_cast<Smem *>(smem_raw);
   const int L = p.L, tid = threadIdx.x;
   const int N = *p.n_cur;
   double *scr = p.scratch + (long)blockIdx.x * p.scr_stride;
