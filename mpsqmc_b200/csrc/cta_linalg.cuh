@@ -1006,15 +1006,13 @@ static __device__ __noinline__ void cta_qr_reg(int m, int n, double *__restrict_
 // (dgeqr2 + dorg2r, with dlarfg's beta = -sign(alpha)*||x||, tau = 0 when the column below the
 // diagonal is zero or m - i == 1).  On exit A holds Q (m x n, orthonormal columns) and R
 // (n x n, ld ldr, upper triangular) holds the triangular factor.  tau: >= n doubles of shared
-// memory; w and red are not used.  Starts and ends with a barrier.
+// memory.  Starts and ends with a barrier.
 //
 // Column j belongs to warp j % kWarps for the whole factorisation: the owner builds reflector j
 // and every warp applies published reflectors to its own columns, so one barrier per column
 // and pass is enough (a warp updates its columns in program order).
 static __device__ __noinline__ void cta_householder_qr(int m, int n, double *A, int lda, double *R, int ldr,
-                                                double *tau, double *w, double *red) {
-  (void)w;
-  (void)red;
+                                                double *tau) {
   if (m <= 64 && n <= 4 * kWarps) {
     cta_qr_reg<2, 4>(m, n, A, lda, R, ldr, tau);
     return;

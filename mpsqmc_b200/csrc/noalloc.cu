@@ -179,9 +179,11 @@ extern "C" int mpsqmc_local_energy_noalloc(const mpsqmc_energy_layout *lay, cons
   if (rc == 0) {
     const bool on_chip = (smem_small + big_doubles) * (long)sizeof(double) <= (long)st->smem_optin;
     const long per_cta = on_chip ? env_doubles : env_doubles + ((big_doubles + 31) & ~31L);
+    // what bond dimensions may take of the array: room for two site tensors and one more environment is part of it
+    const long need = on_chip ? env_doubles : env_doubles + (((8L * pa + 4L * pb) * maxB + 31) & ~31L);
     const size_t smem = sizeof(double) * (size_t)(on_chip ? smem_small + big_doubles : smem_small);
-    if (per_cta > avail) {
-      rc = err(MPSQMC_E_UNSUPPORTED, "bond dimensions need " + std::to_string(per_cta * 8) +
+    if (need > avail) {
+      rc = err(MPSQMC_E_UNSUPPORTED, "bond dimensions need " + std::to_string(need * 8) +
                                          " bytes of scratch per CTA; the static array holds " +
                                          std::to_string(avail * 8));
     } else if ((int)smem > st->smem_optin) {

@@ -890,7 +890,7 @@ __device__ __forceinline__ void general_step(const Dev &args, double *smem_raw) 
             s.QRb[(r + bl * 1) + p.pq * cc] = s.Cen[s.sbC + r + p.pb * cc];
           }
           __syncthreads();
-          cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau, s.wv, s.red);
+          cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau);
           double *Wi = s.W + s.woff[i];
           for (int q = tid; q < bl * br * d; q += kThreads) {
             const int r = q % bl, rest = q / bl, cc = rest % br, sg = rest / br;

@@ -128,14 +128,14 @@ __host__ __device__ inline int padld(int x) {
 // mixed-precision sweep); the small buffers (reductions, closures, PDF) are always FP64.
 template <typename T>
 struct SmemT {
-  T *Lenv, *Cen, *Nxt, *Xb, *Pb, *Qt, *QRb, *Rf;
-  double *red, *tau, *wv, *M, *Cm, *O1, *O2, *pdf, *sc;
+  T *Lenv, *Cen, *Nxt, *Xb, *Pb, *QRb, *Rf;
+  double *red, *tau, *M, *Cm, *O1, *O2, *pdf, *sc;
   float *mlp;   // learned proposal: features (32), hidden (256), partial sums (256), logits (256)
   double *qprop;  // learned proposal: q~ over the grid (G)
   int *bW;      // bond dims of the walker being processed [L+1]
   long *woff;   // its site offsets [L]
   int *wsel;    // the walker index handed out by the work counter
-  int sbC, sbX;  // sigma-block strides of Cen/Nxt and of Xb/Pb/Qt
+  int sbC, sbX;  // sigma-block strides of Cen/Nxt and of Xb/Pb
   int nx;        // blocks of Xb
   // tables of the problem: Dev's, or on-chip copies (read in dependent chains in front of every
   // product, and evicted from the L1 by the environments)
@@ -225,7 +225,6 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   if (engine) off += kTableDoubles + kArgDoubles;
   take(s ? s->red : dummy, 16 * kWarps);
   take(s ? s->tau : dummy, maxB);
-  take(s ? s->wv : dummy, maxB);
   take(s ? s->M : dummy, 16);
   take(s ? s->Cm : dummy, 16);
   take(s ? s->O1 : dummy, 4);
@@ -245,17 +244,15 @@ __host__ __device__ inline long smem_doubles(int L, int maxA, int maxB, int G, i
   }
   take(s ? s->qprop : dummy, mlp ? G : 0);
   take_big(s ? s->Lenv : dummy, (long)pa * maxB);
-  take_big(s ? s->Cen : dummy, (long)pb * maxB * d);
-  take_big(s ? s->Nxt : dummy, (long)pb * maxB * d);
   take_big(s ? s->Xb : dummy, (long)pa * maxB * d);
   take_big(s ? s->Pb : dummy, (long)pa * maxB * kN2);
-  take_big(s ? s->Qt : dummy, (long)pa * maxB);
-  if (engine) {  // the Householder panel and R factor, last: the QR-free sweep goes without them
+  if (engine) {  // site tensors, the Householder panel and R factor
+    take_big(s ? s->Cen : dummy, (long)pb * maxB * d);
+    take_big(s ? s->Nxt : dummy, (long)pb * maxB * d);
     take_big(s ? s->QRb : dummy, (long)pq * maxB);
     take_big(s ? s->Rf : dummy, (long)pb * maxB);
   } else if (s) {
-    s->QRb = nullptr;
-    s->Rf = nullptr;
+    s->Cen = s->Nxt = s->QRb = s->Rf = nullptr;
   }
   if (big_doubles) *big_doubles = boff;
   if (lng_doubles) *lng_doubles = loff;
@@ -352,8 +349,6 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
   const int d = kMaxD;
   off += kTableDoubles + kArgDoubles;
   take(s ? s->red : dummy, 16 * kWarps);
-  take(s ? s->tau : dummy, maxB);
-  take(s ? s->wv : dummy, maxB);
   take(s ? s->M : dummy, 16);
   take(s ? s->Cm : dummy, 16);
   take(s ? s->O1 : dummy, 4);
@@ -389,7 +384,6 @@ __host__ __device__ inline long smem_bytes_f32(int L, int maxA, int maxB, int G,
   take_big(s ? s->Nxt : fdummy, (long)pb * maxB * d);
   take_big(s ? s->Xb : fdummy, (long)pa * maxB * d);
   take_big(s ? s->Pb : fdummy, (long)pa * maxB * kN2);
-  take_big(s ? s->Qt : fdummy, (long)pa * maxB);
   if (s) {
     s->QRb = nullptr;
     s->Rf = nullptr;
@@ -849,7 +843,7 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev args) {
       }
       __syncthreads();
       // move the centre: QR of site i, R into site i+1
-      cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau, s.wv, s.red);
+      cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau);
       gemm_g<0>(br, b2, br, cols(s.Rf, p.pb), 1, rows(s.Nxt, p.pb, s.sbC), d, 1, false, s.Cen, p.pb, 0, s.sbC);
       // site i <- Q
       {
@@ -940,7 +934,7 @@ __global__ void __launch_bounds__(kThreads, 1) set_overlap_kernel(Dev args) {
         for (int sg = 0; sg < d; ++sg) s.QRb[(r + bl * sg) + p.pq * cc] = s.Cen[sg * s.sbC + r + p.pb * cc];
       }
       __syncthreads();
-      cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau, s.wv, s.red);
+      cta_householder_qr(bl * d, br, s.QRb, p.pq, s.Rf, p.pb, s.tau);
       double *Wk = W + s.woff[k];
       for (int q = tid; q < bl * br * d; q += kThreads) {
         const int r = q % bl, rest = q / bl, cc = rest % br, sg = rest / br;
