@@ -665,6 +665,9 @@ static __device__ void env_update(const Dev &p, Smem &s, const double *B, int al
 // ---------------------------------------------------------------------------------------------
 // The walker-step kernel
 // ---------------------------------------------------------------------------------------------
+template <typename T>  // walker_general.cuh
+static __device__ __noinline__ void sample_grid(const Dev &p, SmemT<T> &s, int c, int jq);
+
 __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev args) {
   extern __shared__ double smem_raw[];
   carve_shared<double>(args, smem_raw);
@@ -679,6 +682,7 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev args) {
     const int slot = p.slot_of[w];
     load_walker_dims(p, s, slot);
     double *W = p.walkers + (long)slot * p.wstride;
+    if (tid == 0) s.w = w;
     // ---------------- phase A: right environments ------------------------------------------
     // The walker is read as stored (between steps: left-canonical).  For k = L-1 .. 1:
     //   R[k] = sum_s B_k[s] R[k+1] A_k[s]^T        (a_k x b_k, trial-walker overlap)
@@ -748,8 +752,6 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev args) {
       const int c = p.bond_c[i];
       double num = ov;  // overlap numerator after the bond (no coupling: unchanged)
       if (c >= 0) {
-        const int jq = p.bond_j[i];
-        const double *U = p.tabU + 16 * jq, *Sq = p.tabSq + 4 * jq, *VT = p.tabVT + 16 * jq;
         // left branches P[s + d t] = B_i[s]^T Lenv C[t]
         gemm_g<0>(al, br, bl, cols(s.Lenv, p.pa), 1, rows(s.Cen, p.pb, s.sbC), d, 1, false, s.Xb, p.pa, 0, s.sbX);
         __syncthreads();
@@ -761,66 +763,14 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_kernel(Dev args) {
         gemm_g<0>(a2, br, b2, cols(R2, a2), 1, cols(s.Nxt, p.pb, s.sbC), d, 1, false, s.Xb, p.pa, 0, s.sbX);
         __syncthreads();
         cta_closure16<0>(ar, br, a2, Bj, ar, ar * a2, s.Xb, p.pa, s.sbX, s.Pb, p.pa, s.sbX, s.red, s.M);
-        // C[k + 4 l] = sqrt(s_k s_l) sum_{p,q} U[p + 4k] VT[l + 4q] M[p + 4q]
-        if (tid < 16) {
-          const int k = tid & 3, l = tid >> 2;
-          double acc = 0.0;
-          for (int qq = 0; qq < 4; ++qq) {
-            double inner = 0.0;
-            for (int pp = 0; pp < 4; ++pp) inner += U[pp + 4 * k] * s.M[pp + 4 * qq];
-            acc += inner * VT[l + 4 * qq];
-          }
-          s.Cm[k + 4 * l] = Sq[k] * Sq[l] * acc;
-        }
-        __syncthreads();
-        // PDF over the grid (MPSQMC2.cpp:554-567)
-        const double fac = 4.0 / (ov * p.G);
-        double part = 0.0;
-        for (int g = tid; g < p.G; g += kThreads) {
-          const double *x = p.grid + 4 * g;
-          double v = 0.0;
-          for (int l = 0; l < 4; ++l)
-            for (int r = 0; r < 4; ++r) v += s.Cm[l + 4 * r] * x[l] * x[r];
-          v = fmax(0.0, v);
-          v *= fac;
-          s.pdf[g] = v;
-          part += v;
-        }
-        const double pnorm = cta_sum(part, s.red);
-        const double pinv = 1.0 / pnorm;
-        for (int g = tid; g < p.G; g += kThreads) s.pdf[g] *= pinv;
-        wt *= pnorm;
-        __syncthreads();
+        // C_kl, PDF over the grid, CDF sample, site operators (MPSQMC2.cpp:551-588)
         if (tid == 0) {
-          const double u = p.uni[(long)w * p.nC + c];
-          int count = 0;
-          double cum = s.pdf[0];
-          while ((cum <= u) && (count < p.G - 1)) {
-            count += 1;
-            cum += s.pdf[count];
-          }
-          const double *x = p.grid + 4 * count;
-          double nm = 0.0;
-          for (int l = 0; l < 4; ++l)
-            for (int r = 0; r < 4; ++r) nm += s.Cm[l + 4 * r] * x[l] * x[r];
-          s.sc[1] = 4.0 * nm;
-          s.sc[2] = count;
-          s.sc[3] = u;
-          s.sc[4] = pnorm;
-          // O1(s,t) = sum_k sqrt(4 s_k) x_k U[s + 2(t + 2k)], O2(s,t) = sum_l sqrt(4 s_l) x_l VT[l + 4(s + 2t)]
-          for (int q = 0; q < 4; ++q) {
-            double o1 = 0.0, o2 = 0.0;
-            for (int k = 0; k < 4; ++k) {
-              const double pf = 2.0 * Sq[k] * x[k];  // sqrt(4 s_k) x_k
-              o1 += pf * U[q + 4 * k];
-              o2 += pf * VT[k + 4 * q];
-            }
-            s.O1[q] = o1;
-            s.O2[q] = o2;
-          }
+          s.sc[kScOv] = ov;
+          s.sc[kScWt] = wt;
         }
-        __syncthreads();
-        num = s.sc[1];
+        sample_grid(p, s, c, p.bond_j[i]);
+        num = s.sc[kScOv];
+        wt = s.sc[kScWt];
         // apply O1 to the centre (into the QR layout), O2 to site j in place
         for (int q = tid; q < bl * br; q += kThreads) {
           const int r = q % bl, cc = q / bl;
