@@ -106,6 +106,7 @@ struct mpsqmc_ctx {
   size_t smem_bytes_free = 0;
   long fwoff = 0;
   int free_threads = mq::kThreads, max_ctas_free = 1;
+  int sm_places = 1 << 20;              // walkers per SM at most
   int sm_count = 1, max_ctas = 1;
   // mixed-precision sweep (FP32 work buffers, TF32 tensor cores): its own shared memory and grid
   int precision = MPSQMC_PRECISION_FP64;
@@ -402,9 +403,10 @@ bool mlp_on(const mpsqmc_ctx *c) {
 //   64, 16-64, 444 walkers (6x6 lattice):               512x1 69     256x2 60     128x3 77
 //   16, 16, 128 walkers (L = 16 chain, one per SM):     512x1 0.50   256x1 0.42   128x1 0.55
 //   256, 64, 148 walkers (8x8 lattice, one per SM):     512x1 503    256x1 716
-void free_shape(const mpsqmc_ctx *c, int *threads, int *ctas) {
+// places: walkers that an SM (its shared memory, the device's memory for their scratch) has room for.
+void free_shape(const mpsqmc_ctx *c, int places, int *threads, int *ctas) {
   const long a = (long)c->maxA * c->maxB;
-  const int per_sm = std::max(1, (c->Ndesired + c->sm_count - 1) / c->sm_count);
+  const int per_sm = std::min(places, std::max(1, (c->Ndesired + c->sm_count - 1) / c->sm_count));
   int th = 512, n = 1;
   if (a <= 64) th = 64, n = 8;
   else if (a < 2048 || (a < 4096 && !c->nn)) th = 128, n = 3;
@@ -426,45 +428,53 @@ void free_shape(const mpsqmc_ctx *c, int *threads, int *ctas) {
 // The PDF and the walker's dims, written by the sweep, stay on chip while a CTA can hold them.
 constexpr size_t kSmallTable = 4096;
 int layout_free(mpsqmc_ctx *c, bool force_global) {
-  int threads = 0, ctas = 0;
-  free_shape(c, &threads, &ctas);
-  const size_t share =
-      force_global ? 0 : std::min(c->smem_optin, c->smem_sm / ctas - 1024 - mq::kOpBytes);
-  auto bytes = [&](const mq::FreeLayout &f, long *big) {
-    return sizeof(double) * (size_t)mq::free_doubles(c->L, c->nC, c->maxB, c->G, c->nJ, c->pa, c->pb, f, nullptr, nullptr,
-                                                     nullptr, big);
-  };
-  mq::FreeLayout f{0u, 2};
-  auto add = [&](int k, size_t limit) {
-    const mq::FreeLayout g{f.place | 1u << k, 2};
-    if (bytes(g, nullptr) <= limit) f = g;
-  };
-  for (int k : {mq::kBufPdf, mq::kBufDims}) add(k, c->smem_optin);
-  for (int k : {mq::kBufSites, mq::kBufCoup, mq::kBufTab})
-    if (bytes({1u << k, 2}, nullptr) - bytes({0u, 2}, nullptr) <= kSmallTable) add(k, force_global ? c->smem_optin : share);
-  const mq::FreeLayout small = f;
-  const unsigned matrix = (1u << mq::kNumMat) - 1;
-  for (int nx : {8, 6, 4})
-    if (f.nx == 2 && bytes({small.place | matrix, nx}, nullptr) <= share) f = {small.place | matrix, nx};
-  if (f.nx == 2)
-    for (int k = 0; k < mq::kNumMat; ++k) add(k, share);
-  for (int k : {mq::kBufCoup, mq::kBufSites, mq::kBufTab}) {
-    const mq::FreeLayout g{f.place | 1u << k, f.nx};
-    if (bytes(g, nullptr) <= share) f = g;
+  for (int places = c->sm_places;;) {
+    int threads = 0, ctas = 0;
+    free_shape(c, places, &threads, &ctas);
+    const size_t share =
+        force_global ? 0 : std::min(c->smem_optin, c->smem_sm / ctas - 1024 - mq::kOpBytes);
+    auto bytes = [&](const mq::FreeLayout &f, long *big) {
+      return sizeof(double) * (size_t)mq::free_doubles(c->L, c->nC, c->maxB, c->G, c->nJ, c->pa, c->pb, f, nullptr, nullptr,
+                                                       nullptr, big);
+    };
+    mq::FreeLayout f{0u, 2};
+    auto add = [&](int k, size_t limit) {
+      const mq::FreeLayout g{f.place | 1u << k, 2};
+      if (bytes(g, nullptr) <= limit) f = g;
+    };
+    for (int k : {mq::kBufPdf, mq::kBufDims}) add(k, c->smem_optin);
+    for (int k : {mq::kBufSites, mq::kBufCoup, mq::kBufTab})
+      if (bytes({1u << k, 2}, nullptr) - bytes({0u, 2}, nullptr) <= kSmallTable) add(k, force_global ? c->smem_optin : share);
+    const mq::FreeLayout small = f;
+    const unsigned matrix = (1u << mq::kNumMat) - 1;
+    for (int nx : {8, 6, 4})
+      if (f.nx == 2 && bytes({small.place | matrix, nx}, nullptr) <= share) f = {small.place | matrix, nx};
+    if (f.nx == 2)
+      for (int k = 0; k < mq::kNumMat; ++k) add(k, share);
+    for (int k : {mq::kBufCoup, mq::kBufSites, mq::kBufTab}) {
+      const mq::FreeLayout g{f.place | 1u << k, f.nx};
+      if (bytes(g, nullptr) <= share) f = g;
+    }
+    long big = 0;
+    const size_t smem = bytes(f, &big);
+    int occ = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mq::walker_step_kernel_fp64<false>, threads, smem));
+    const long fwoff = (c->scr_base + 31) & ~31L, stride = std::max(c->scr_stride, (fwoff + big + 31) & ~31L);
+    // several walkers per SM only where their scratch leaves most of the device memory to the populations
+    int n = std::max(1, std::min(occ, ctas));
+    while (n > 1 && (size_t)n * c->sm_count * stride * sizeof(double) > c->total_mem / 16) --n;
+    if (n < ctas) {  // room for fewer than the rule asks for: threads and layout for those
+      places = n;
+      continue;
+    }
+    c->fl = f;
+    c->fwoff = fwoff;
+    c->scr_stride = stride;
+    c->smem_bytes_free = smem;
+    c->free_threads = threads;
+    c->max_ctas_free = n * c->sm_count;
+    return 0;
   }
-  c->fl = f;
-  long big = 0;
-  c->smem_bytes_free = bytes(f, &big);
-  c->fwoff = (c->scr_base + 31) & ~31L;
-  c->scr_stride = std::max(c->scr_stride, (c->fwoff + big + 31) & ~31L);
-  c->free_threads = threads;
-  int occ = 1;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mq::walker_step_kernel_fp64<false>, threads, c->smem_bytes_free));
-  // several walkers per SM only where their scratch leaves most of the device memory to the populations
-  int n = std::max(1, std::min(occ, ctas));
-  while (n > 1 && (size_t)n * c->sm_count * c->scr_stride * sizeof(double) > c->total_mem / 16) --n;
-  c->max_ctas_free = n * c->sm_count;
-  return 0;
 }
 
 // Every kernel's dynamic shared memory may reach the device's limit: the attribute belongs to the

@@ -111,3 +111,8 @@ def test_grid_beyond_the_limit_is_refused():
     with pytest.raises(MpsqmcError) as e:
         Engine(**kw)
     assert e.value.code == E_UNSUPPORTED
+
+
+def test_step_where_shared_memory_holds_fewer_walkers_than_the_shape():
+    """A grid whose PDF takes most of a CTA's share: fewer CTAs per SM than the bonds alone would have."""
+    check_step(*make("chain:10", 4, 9000, 1300, False))
