@@ -106,7 +106,7 @@ struct mpsqmc_ctx {
   size_t smem_bytes_free = 0;
   long fwoff = 0;
   int free_threads = mq::kThreads, max_ctas_free = 1;
-  int sm_places = 1 << 20;              // walkers per SM at most
+  int sm_places = 1 << 20;              // walkers per SM at most: one where device memory is short
   int sm_count = 1, max_ctas = 1;
   // mixed-precision sweep (FP32 work buffers, TF32 tensor cores): its own shared memory and grid
   int precision = MPSQMC_PRECISION_FP64;
@@ -321,6 +321,20 @@ size_t scratch_doubles(const mpsqmc_ctx *c) {
 
 int layout_workspace(mpsqmc_ctx *c, bool force_global);
 
+// The scratch, of one walker per SM in the QR-free FP64 sweep where that of several does not fit into the
+// device's memory (a population that leaves no room for more).
+int alloc_scratch(mpsqmc_ctx *c, bool force_global) {
+  if (cudaMalloc((void **)&c->d_scratch, sizeof(double) * scratch_doubles(c)) == cudaSuccess) return 0;
+  cudaGetLastError();
+  c->d_scratch = nullptr;
+  if (c->max_ctas_free > c->sm_count) {
+    c->sm_places = 1;
+    const int rc = layout_workspace(c, force_global);
+    if (rc) return rc;
+  }
+  return dalloc(&c->d_scratch, scratch_doubles(c));
+}
+
 // Recompute the work-buffer layout (after an option that changes it) and grow the scratch if needed.
 int relayout(mpsqmc_ctx *c, bool force_global) {
   CK(cudaSetDevice(c->device));
@@ -330,8 +344,7 @@ int relayout(mpsqmc_ctx *c, bool force_global) {
   if (rc) return rc;
   if (scratch_doubles(c) > before) {
     cudaFree(c->d_scratch);
-    c->d_scratch = nullptr;
-    if (dalloc(&c->d_scratch, scratch_doubles(c))) return MPSQMC_E_CUDA;
+    return alloc_scratch(c, force_global);
   }
   return 0;
 }
@@ -797,7 +810,7 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
         dalloc(&c->d_bond_j, L - 1) | dalloc(&c->d_bondJ, L - 1) | dalloc(&c->d_tabU, 16 * c->nJ) |
         dalloc(&c->d_tabS, 4 * c->nJ) | dalloc(&c->d_tabVT, 16 * c->nJ) | dalloc(&c->d_grid, 4 * c->G) |
         dalloc(&c->d_tabSq, 4 * c->nJ) |
-        dalloc(&c->d_scratch, scratch_doubles(c)) | dalloc(&c->d_err, 1) | dalloc(&c->d_trial32, to) |
+        dalloc(&c->d_err, 1) | dalloc(&c->d_trial32, to) |
         dalloc(&c->d_mt, 1) | dalloc(&c->d_sd, 1) | dalloc(&c->d_cp_j, c->nC) | dalloc(&c->d_cp_q, c->nC) |
         dalloc(&c->d_site_c0, L + 1) | dalloc(&c->d_ech_off, L + 1) | dalloc(&c->d_ech_slot, ech_slot.size()) |
         dalloc(&c->d_ech_cont, ech_cont.size()) | dalloc(&c->d_eopen, L) | dalloc(&c->d_ech_J, ech_J.size()) |
@@ -805,6 +818,7 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
         dalloc(&c->d_ctr, mq::kNumCtr) | dalloc(&c->d_term_slot, term_slot.size()) |
         dalloc(&c->d_term_site, term_site.size()) | dalloc(&c->d_term_op, term_op.size()) |
         dalloc(&c->d_term_pref, term_pref.size()) | dalloc(&c->d_changed, cap);
+  if (!rc) rc = alloc_scratch(c, false);  // last: it can do with less
   if (rc) return bail(MPSQMC_E_CUDA);
   if (cudaMallocHost((void **)&c->h_sd, sizeof(mq::StepDev)) != cudaSuccess ||
       cudaMallocHost((void **)&c->h_err, sizeof(int)) != cudaSuccess)
@@ -1311,8 +1325,19 @@ static int ensure_batched(mpsqmc_ctx *c) {
   // buffers for the whole slot capacity when they fit in half the free memory, else for 1.5x the
   // target population (a step with more walkers then stops with MPSQMC_E_CAPACITY)
   size_t free_b = 0, total_b = 0;
-  CK(cudaMemGetInfo(&free_b, &total_b));
   pr.capacity = c->capacity;
+  CK(cudaMemGetInfo(&free_b, &total_b));
+  if (mq::bs::bytes_needed(pr) > free_b / 2 && c->max_ctas_free > c->sm_count) {
+    // the FP64 sweep, which does not run here, gives back its scratch for more than one walker per SM
+    c->sm_places = 1;
+    cudaFree(c->d_scratch);
+    c->d_scratch = nullptr;
+    int rc = layout_workspace(c, c->workspace == MPSQMC_WORKSPACE_GLOBAL);
+    if (!rc) rc = alloc_scratch(c, c->workspace == MPSQMC_WORKSPACE_GLOBAL);
+    if (rc) return rc;
+    drop_graphs(c);
+    CK(cudaMemGetInfo(&free_b, &total_b));
+  }
   if (mq::bs::bytes_needed(pr) > free_b / 2)
     pr.capacity = std::min(c->capacity, std::max(64, (3 * c->Ndesired + 1) / 2));
   if (mq::bs::bytes_needed(pr) > free_b * 9 / 10)
@@ -1807,6 +1832,11 @@ int mpsqmc_set_option(mpsqmc_ctx *c, int option, long value) {
         CK(cudaStreamSynchronize(c->stream));
         mq::bs::destroy(c->bplan);
         c->bplan = nullptr;
+      }
+      if (!tc_sweep(c) && c->sm_places == 1) {  // there may be room for more again
+        c->sm_places = 1 << 20;
+        const int rc = relayout(c, c->workspace == MPSQMC_WORKSPACE_GLOBAL);
+        if (rc) return rc;
       }
       break;
     case MPSQMC_OPT_PROPOSAL:
