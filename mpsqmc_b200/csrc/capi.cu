@@ -106,6 +106,7 @@ struct mpsqmc_ctx {
   size_t smem_bytes_free = 0;
   long fwoff = 0;
   int free_threads = mq::kThreads, max_ctas_free = 1;
+  int population = 0;                   // walkers that the launch shape is for (Ndesired)
   int sm_places = 1 << 20;              // walkers per SM at most: one where device memory is short
   int sm_count = 1, max_ctas = 1;
   // mixed-precision sweep (FP32 work buffers, TF32 tensor cores): its own shared memory and grid
@@ -419,7 +420,7 @@ bool mlp_on(const mpsqmc_ctx *c) {
 // places: walkers that an SM (its shared memory, the device's memory for their scratch) has room for.
 void free_shape(const mpsqmc_ctx *c, int places, int *threads, int *ctas) {
   const long a = (long)c->maxA * c->maxB;
-  const int per_sm = std::min(places, std::max(1, (c->Ndesired + c->sm_count - 1) / c->sm_count));
+  const int per_sm = std::min(places, std::max(1, (c->population + c->sm_count - 1) / c->sm_count));
   int th = 512, n = 1;
   if (a <= 64) th = 64, n = 8;
   else if (a < 2048 || (a < 4096 && !c->nn)) th = 128, n = 3;
@@ -710,7 +711,7 @@ int mpsqmc_create(const mpsqmc_config *cfg, mpsqmc_ctx **out) {
   c->nC = cfg->nC;
   c->G = cfg->G;
   c->nJ = cfg->nJ;
-  c->Ndesired = cfg->Ndesired;
+  c->Ndesired = c->population = cfg->Ndesired;
   c->capacity = cfg->capacity;
   c->dtau = cfg->dtau;
   c->h = cfg->h;
@@ -1606,9 +1607,11 @@ int mpsqmc_autotune(mpsqmc_ctx *c, int steps, int *best_sweep, int *best_workspa
     }
   }
   // measure on the first k walkers, with the population state saved and restored around every
-  // trial: two waves of one CTA per SM for the per-walker sweeps; for the tcgen05 sweep, whose
-  // tile counts grow with the population, up to 1024 walkers
-  const int N = c->n_cur, k = std::min(N, tc ? 1024 : 2 * c->sm_count), cap = c->capacity, L = c->L;
+  // trial: two waves of the CTAs that a launch has for the per-walker sweeps (their shape is the
+  // whole population's, c->population); for the tcgen05 sweep, whose tile counts grow with the
+  // population, up to 1024 walkers
+  const int N = c->n_cur, k = std::min(N, tc ? 1024 : 2 * std::max(c->max_ctas, c->max_ctas_free)), cap = c->capacity,
+            L = c->L;
   std::vector<int> slots(N), h_free(cap), wd((size_t)cap * (L + 1));
   std::vector<long> wf((size_t)cap * L);
   std::vector<double> wt(cap), ov(cap), eh(cap);
