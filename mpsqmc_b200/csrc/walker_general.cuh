@@ -808,7 +808,9 @@ __device__ __forceinline__ void general_step(const Dev &args, double *smem_raw) 
       if (i + 1 < L) {
         const int br = s.bW[i + 1];
         prefetch_l2(s.W + s.woff[i + 1], (long)br * s.bW[i + 2] * d);
-        if constexpr (ZB) prefetch_l2(s.scr + s.zoff[i + 1], 4L * s.aT[i + 1] * br);
+        if constexpr (ZB)
+          for (int q = 0; q < kN2; ++q)
+            prefetch_l2(s.scr + s.zoff[i + 1] + (long)q * s.aT[i + 1] * s.bS[i + 1], (long)s.aT[i + 1] * br);
       }
       // Pb still holds the last coupling's left branches at cut i+1 (its partner was i+1, so they
       // were not carried further, and the trace did not use Pb as scratch)
@@ -935,7 +937,7 @@ __global__ void __launch_bounds__(kThreads, 1) walker_step_general_kernel(Dev p)
 }
 
 // Mixed precision: FP32 work buffers, TF32 tensor cores (NP passes), always QR-free.  Half the
-// shared memory of the FP64 sweep, so two CTAs fit on an SM where the FP64 sweep fits one.
+// matrix buffers' bytes, so two CTAs of 256 threads fit on an SM where they would be one in FP64.
 template <int NP, bool ZB>
 __global__ void __launch_bounds__(kThreads, 2) walker_step_mixed_kernel(Dev p) {
   extern __shared__ double smem_raw[];
