@@ -351,7 +351,7 @@ __device__ __forceinline__ void cta_gemm_groups() {
 // The same product for small matrices, one output element per thread and round: a tile's set-up,
 // some 300 dependent instructions, costs more than the products of up to 8 x 8 x 8 elements do this
 // way (the bonds of the smallest walks, and the ends of every chain).
-__host__ __device__ constexpr bool small_product(int M, int N, int K) { return (long)M * N * K <= 512; }
+__host__ __device__ constexpr bool small_product(int M, int N, int K) { return M * N <= 512 && M * N * K <= 512; }
 static_assert(!small_product(4096, 128, 4096), "the product of the sizes exceeds an int");
 template <typename T>
 static __device__ __noinline__ void cta_gemm_small() {
