@@ -277,11 +277,18 @@ __device__ __forceinline__ void dmma_tiles(const volatile GemmOp &op, Epi &epi) 
   }
 }
 
-// Pieces per tile: the wider tiles where they still give every warp one.
+// Pieces per tile: the wider tiles where they still give every warp one.  A CTA of kMaxWarps warps has its
+// SM to itself, and nothing fills the warps that wait for a last round of tiles: there the pieces
+// take the fewest rounds, a tile's work being its pieces and one more (its set-up and left factor):
+// four for more blocks than warps, but for 33 to 48 blocks two (three rounds of 3, not two of 5); two
+// for more than half as many (one round of 3, not two of 2).  Measured (ms a step, few walkers): 6x6
+// lattice, 64/48, 20 walkers 26.2, now 19.4; two rows of 8, 96/48, 148 walkers 9.4, now 8.6.
 template <typename T>
 __device__ __forceinline__ int tile_pieces(const volatile GemmOpT<T> &op) {
   const int N = op.N, blocks = op.GM * ((op.M + 15) >> 4) * op.GN * ((N + 15) >> 4), nw = blockDim.x >> 5;
-  return blocks >= 2 * nw ? 4 : blocks >= nw && N > 8 ? 2 : 1;
+  const bool alone = nw == kMaxWarps;
+  if (alone ? blocks > kMaxWarps && (unsigned)(blocks - 2 * kMaxWarps - 1) >= (unsigned)kMaxWarps : blocks >= 2 * nw) return 4;
+  return blocks >= (alone ? kMaxWarps / 2 + 1 : nw) && N > 8 ? 2 : 1;
 }
 
 // One function per tile shape: together in one body they share what can be computed in front of the
