@@ -427,6 +427,23 @@ __device__ __forceinline__ void take_point(const Dev &p, SmemT<T> &s, int jq, in
   }
 }
 
+// The point where the warp's scan (sample_grid) found none (from == G) or one of probability zero (from): the
+// next of nonzero probability, or the last one; and where the sum of the PDF is zero, infinite or no
+// number, the point at which the serial scan's comparisons end.
+static __device__ __noinline__ int rare_point(const double *pdf, int G, int per, int from, double pinv, double u) {
+  auto at = [&](int g) { return pdf[32 * (g % per) + g / per]; };
+  int g = from;
+  if (!(pinv > 0.0 && pinv <= DBL_MAX)) {
+    g = 0;
+    for (double cum = at(0) * pinv; cum <= u && g < G - 1; cum += at(g) * pinv) ++g;
+    return g;
+  }
+  while (g < G && at(g) == 0.0) ++g;
+  if (g >= G)
+    for (g = G - 1; g > 0 && at(g) == 0.0;) --g;
+  return g;
+}
+
 // C_kl from the closures, PDF over the grid, weight update, CDF sample with the walker's uniform
 // for coupling c, and the site operators O1, O2 (MPSQMC2.cpp:551-588, MPSstate.cpp:575-633).
 // The CDF scan is one warp's: lane k holds the run of grid points from k*per on (stored per-major,
@@ -471,24 +488,13 @@ static __device__ __noinline__ void sample_grid(const Dev &p, SmemT<T> &s, int c
     if (lane == 0) at = 0.0;
     int hit = per;
     for (int i = 0; i < per; ++i) {
-      const double v = s.pdf[32 * i + lane];
-      at += v;
-      if (hit == per && at * pinv > u && __double2hiint(v) != 0) hit = i;
+      at += s.pdf[32 * i + lane];
+      if (hit == per && at * pinv > u) hit = i;
     }
     const unsigned who = __ballot_sync(full, hit < per);
-    int count = 0;
-    if (!(pinv > 0.0 && pinv <= DBL_MAX)) {  // a sum that is zero, infinite or no number: as the serial scan ends
-      auto pdf = [&](int g) { return s.pdf[32 * (g % per) + g / per] * pinv; };
-      for (double cum = pdf(0); cum <= u && count < p.G - 1; cum += pdf(count)) ++count;
-    } else if (who) {
-      const int src = __ffs(who) - 1;
-      count = min(p.G - 1, src * per + __shfl_sync(full, hit, src));
-    } else {  // u beyond the last sum by rounding: the last point of nonzero probability
-      int last = -1;
-      for (int i = 0; i < per; ++i)
-        if (s.pdf[32 * i + lane] > 0.0) last = lane * per + i;
-      count = __reduce_max_sync(full, last);
-    }
+    const int src = __ffs(who) - 1, h = __shfl_sync(full, hit, src & 31);
+    int count = src * per + h;
+    if (!who || s.pdf[32 * h + src] == 0.0) count = rare_point(s.pdf, p.G, per, who ? count : p.G, pinv, u);
     take_point(p, s, jq, count, u, pnorm);
   }
   __syncthreads();
