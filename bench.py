@@ -588,7 +588,8 @@ def main():
     if rank == 0:
         prof_traffic = None
         kname = "walker_step_kernel" if args.sweep == "nearest" else (
-            "tc_gemm_kernel" if tc else ("walker_step_mixed_kernel" if mixed else "walker_step_general_kernel"))
+            "tc_gemm_kernel" if tc else "walker_step_mixed_kernel" if mixed else
+            "walker_step_general_kernel" if training else "walker_step_kernel_fp64")
         tp = os.path.join(ROOT, "profiles", f"{kname}_{wl.name}_traffic.json")
         if os.path.exists(tp):
             prof_traffic = json.load(open(tp)).get("bytes_per_step_per_walker")

@@ -409,14 +409,25 @@ bool mlp_on(const mpsqmc_ctx *c) {
 // The QR-free FP64 sweep's threads per walker and walkers per SM.  A walker's sweep is a dependent chain of
 // small operations, so walkers that share an SM fill one another's waits; more threads per walker
 // only pay where its products fill them, or where there is no second walker for the SM.  128
-// registers a thread: 512 threads per SM.  Measured (ms per step, threads x walkers per SM):
-//   D_T = 4, D_W = 2, 1000 walkers (L = 20 chain):      256x1 2.84   128x4 0.95   64x8 0.60
-//   16, 8, 740 walkers (6x3 lattice):                   256x1 6.02   128x3 3.27   64x8 3.74
-//   64, 32, 1024 walkers (L = 64 chain):                512x1 32.1   256x2 24.8   128x3 31.6
-//   64, 32, 444 walkers (8x8 lattice):                  512x1 107    256x2 96     128x3 82
-//   64, 16-64, 444 walkers (6x6 lattice):               512x1 69     256x2 60     128x3 77
-//   16, 16, 128 walkers (L = 16 chain, one per SM):     512x1 0.50   256x1 0.42   128x1 0.55
-//   256, 64, 148 walkers (8x8 lattice, one per SM):     512x1 503    256x1 716
+// registers a thread: 512 threads per SM.  Measured (ms of the walker kernel per step, threads x
+// walkers per SM; a = D_T D_W):
+//   a = 8      4/2, 1000 walkers (L = 20 chain):            256x1 2.84   128x4 0.95   64x8 0.60
+//   64         8/8, 1000 walkers (6x3 lattice):             256x2 5.07   128x3 4.25   64x8 2.94
+//   128        16/8, 1000 walkers (6x3 lattice):            256x2 5.73   128x3 4.64   64x8 3.81
+//   256        16/16, 444 walkers (L = 24 chain):           512x1 2.03   256x2 1.50   128x3 0.82   64x8 1.19
+//   768        32/24, 444 walkers (6x3 lattice):            512x1 7.15   256x2 6.77   128x3 5.22
+//   2025       45/45, 444 walkers (6x3 lattice):            512x1 23.7   256x2 23.3   128x3 17.6
+//   2048       64/32, 1024 walkers (L = 64 chain):          512x1 32.1   256x2 24.8   128x3 31.6
+//   2048       64/32, 444 walkers (6x6 lattice):            512x1 41.1   256x2 36.7   128x3 31.1
+//   3072       64/48, 444 walkers (6x6 lattice):            512x1 84.7   256x2 70.3   128x3 56.3
+//   4096       64/64, 444 walkers (6x6 lattice):            512x1 79.4   256x2 79.1   128x3 99.0
+//   6144       128/48, 444 walkers (8x2 lattice):           512x1 32.5   256x2 28.2   128x3 31.1
+//   12800      200/64, 444 walkers (8x2 lattice):           512x1 44.1   256x2 55.5   128x3 60.5
+//   one walker per SM: 16/16 (L = 16 chain)  512x1 0.50  256x1 0.42  128x1 0.55;  32/24 (6x3)  512x1 2.37
+//   256x1 2.34  128x1 2.99;  64/32 (6x6)  512x1 13.6  256x1 14.6;  256/64 (8x8)  512x1 503  256x1 716
+// Where another shape is faster: 64x8 for a = 65 to 300 with seven walkers per SM (16/16, 1000 walkers,
+// L = 24 chain: 1.24, 128x3 2.39), 512x1 from a = 8192 on when 256x2 leaves the SM's second round half
+// empty (the row of 12800), and 512x1 for chains of a about 2000 with one walker per SM (1.88, 256x1 2.19).
 // places: walkers that an SM (its shared memory, the device's memory for their scratch) has room for.
 void free_shape(const mpsqmc_ctx *c, int places, int *threads, int *ctas) {
   const long a = (long)c->maxA * c->maxB;

@@ -286,7 +286,7 @@ __device__ __forceinline__ void dmma_tiles(const volatile GemmOp &op, Epi &epi) 
 template <typename T>
 __device__ __forceinline__ int tile_pieces(const volatile GemmOpT<T> &op) {
   const int N = op.N, blocks = op.GM * ((op.M + 15) >> 4) * op.GN * ((N + 15) >> 4), nw = blockDim.x >> 5;
-  const bool alone = nw == kMaxWarps;
+  const bool alone = std::is_same<T, double>::value && nw == kMaxWarps;  // (the TF32 sweep has eight warps)
   if (alone ? blocks > kMaxWarps && (unsigned)(blocks - 2 * kMaxWarps - 1) >= (unsigned)kMaxWarps : blocks >= 2 * nw) return 4;
   return blocks >= (alone ? kMaxWarps / 2 + 1 : nw) && N > 8 ? 2 : 1;
 }
@@ -427,8 +427,9 @@ __device__ __forceinline__ void tf32_split(float x, uint32_t &head, uint32_t &ta
 // Each chunk is summed in accumulators of its own, the small products first, and these are then added
 // up in FP32: the tensor cores' sums truncate, and a chain over all of K costs accuracy.  Measured on
 // the L = 64 chain (D_T = 64, D_W = 32, 1,024 walkers): 25.2 ms a step with 16x16 blocks, one
-// 4-byte load per element and one chain over K, 20.7 ms with these tiles; error against 64 bits
-// 8.2e-6 before, 1.1e-5 with the long chain, 5.5e-6 as it is.
+// 4-byte load per element and one chain over K, 20.7 ms with these tiles (19.6 ms with the reads of
+// the elementwise loops in flight together).  Error against 64 bits on one population: 8.2e-6 before,
+// 1.1e-5 with the long chain, 5.5e-6 as it is; on another 8.2e-7 before and 7.5e-7 as it is.
 template <int PASSES, int NP, bool KA, bool KB, bool VA, bool VB, class Epi>
 __device__ __forceinline__ void tf32_tiles(const volatile GemmOpT<float> &op, Epi &epi) {
   constexpr int kW = NP == 1 ? 8 : 16, kBlk = NP == 1 ? 1 : NP / 2;
